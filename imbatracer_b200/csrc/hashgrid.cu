@@ -208,49 +208,27 @@ __global__ void scatter_kernel(const float* __restrict__ pos, int stride, int n,
     }
 }
 
-// One query per thread (the search itself is grid_query_knn, hashgrid_query.cuh).
-__global__ void query_kernel(const float4* __restrict__ sorted, const int* __restrict__ ends,
-                             const float* __restrict__ prm, uint32_t table, const float* __restrict__ queries,
-                             int nq, int k, int* __restrict__ out_ids, int* __restrict__ out_count,
-                             float* __restrict__ out_d2) {
-    __shared__ float sp[10];
-    if (threadIdx.x < 10) sp[threadIdx.x] = prm[threadIdx.x];
-    __syncthreads();
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= nq) return;
-    const float qx = queries[3 * (size_t)q + 0], qy = queries[3 * (size_t)q + 1], qz = queries[3 * (size_t)q + 2];
-    float dist[kMaxK];
-    int ids[kMaxK];
-    const int count = grid_query_knn(sorted, ends, sp, table, qx, qy, qz, k, dist, ids);
-    out_count[q] = count;
-    int* o = out_ids + (size_t)q * k;
-    for (int i = 0; i < k; ++i) o[i] = i < count ? ids[i] : -1;
-    if (out_d2) {
-        float* od = out_d2 + (size_t)q * k;
-        for (int i = 0; i < k; ++i) od[i] = i < count ? dist[i] : 0.0f;
-    }
-}
-
-// One warp per query (k <= 32; the search is grid_query_knn_warp): lane i writes entry i.
-__global__ void __launch_bounds__(128) query_warp_kernel(const float4* __restrict__ sorted,
+// One warp per query (the search is grid_query_knn_warp).
+template <int kCap>
+__global__ void __launch_bounds__(128, 10) query_warp_kernel(const float4* __restrict__ sorted,
                                                          const int* __restrict__ ends, const float* __restrict__ prm,
                                                          uint32_t table, const float* __restrict__ queries, int nq,
                                                          int k, int* __restrict__ out_ids, int* __restrict__ out_count,
                                                          float* __restrict__ out_d2) {
     __shared__ float sp[10];
+    __shared__ KnnScratch<kCap> scratch[4];
     if (threadIdx.x < 10) sp[threadIdx.x] = prm[threadIdx.x];
     __syncthreads();
     const long long q = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (q >= nq) return;   // uniform across the warp
     const int lane = threadIdx.x & 31;
     const float qx = queries[3 * q + 0], qy = queries[3 * q + 1], qz = queries[3 * q + 2];
-    float my_d;
-    int my_id;
-    const int count = grid_query_knn_warp(sorted, ends, sp, table, qx, qy, qz, k, my_d, my_id);
+    KnnScratch<kCap>& s = scratch[threadIdx.x >> 5];
+    const int count = grid_query_knn_warp<kCap>(sorted, ends, sp, table, qx, qy, qz, k, s);
     if (lane == 0) out_count[q] = count;
-    if (lane < k) {
-        out_ids[q * k + lane] = lane < count ? my_id : -1;
-        if (out_d2) out_d2[q * k + lane] = lane < count ? my_d : 0.0f;
+    for (int i = lane; i < k; i += 32) {
+        out_ids[q * k + i] = i < count ? s.id[i] : -1;
+        if (out_d2) out_d2[q * k + i] = i < count ? __uint_as_float(s.d2[i]) : 0.0f;
     }
 }
 
@@ -383,16 +361,10 @@ int imbart_hashgrid_query(const imbart_hashgrid* g, const float* queries, int nq
     int prev = 0;
     cudaGetDevice(&prev);
     cudaSetDevice(g->device);
-    if (k <= 32) {
-        // One warp per query: coalesced photon loads and the list in registers.
-        const long long grid = ((long long)nq * 32 + 127) / 128;
-        query_warp_kernel<<<(unsigned)grid, 128, 0, (cudaStream_t)stream>>>(
-            g->sorted, g->cell_ends, g->params, (uint32_t)g->table, queries, nq, k, out_ids, out_counts, out_d2);
-    } else {
-        const int grid = (nq + 127) / 128;
-        query_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(g->sorted, g->cell_ends, g->params, (uint32_t)g->table,
-                                                             queries, nq, k, out_ids, out_counts, out_d2);
-    }
+    const auto kernel = k <= 32 ? query_warp_kernel<kKnnCapSmall> : query_warp_kernel<kKnnCapLarge>;
+    const long long blocks = ((long long)nq * 32 + 127) / 128;
+    kernel<<<(unsigned)blocks, 128, 0, (cudaStream_t)stream>>>(g->sorted, g->cell_ends, g->params, (uint32_t)g->table,
+                                                               queries, nq, k, out_ids, out_counts, out_d2);
     note_launches(1);
     const bool good = ok(cudaGetLastError(), "hash grid query");
     cudaSetDevice(prev);

@@ -512,122 +512,65 @@ __device__ __forceinline__ bool vcm_connect_one(const VcmParams& p, int cam_path
     return true;
 }
 
-// VCMIntegrator::vertex_merging (vcm.cpp:571-611): the k nearest photons of the grid, one
-// thread per query (the path for k > 32; vcm_merge_warp_kernel serves k <= 32).
-__device__ __forceinline__ V3 vcm_merge(const VcmParams& p, V3 thr, float dVCM, float dVM, const Isect& is,
-                                        const Bsdf& bsdf) {
-    float dist[kGridMaxK];
-    int ids[kGridMaxK];
-    float prm[10];
-    for (int k = 0; k < 10; ++k) prm[k] = __ldg(p.grid_params + k);
-    const int k = p.num_knn;
-    const int count = grid_query_knn(p.grid_sorted, p.grid_ends, prm, p.grid_table, is.pos.x, is.pos.y, is.pos.z, k,
-                                     dist, ids);
-    float radius_sqr = p.pm_radius * p.pm_radius;
-    if (count == k) {
-        const float4 q = __ldg(p.cache + 7 * (size_t)ids[k - 1]);
-        const V3 d = v3(q) - is.pos;
-        radius_sqr = dot(d, d);
-    }
-    V3 contrib(0.0f);
-    for (int i = 0; i < count; ++i) {
-        const float4* v = p.cache + 7 * (size_t)ids[i];
-        const float4 q0 = __ldg(v), q1 = __ldg(v + 1), q3 = __ldg(v + 3), q4 = __ldg(v + 4), q6 = __ldg(v + 6);
-        const V3 photon_in_dir = v3(q1);
-        const V3 bsdf_value = bsdf.eval(is.out_dir, photon_in_dir);
-        const float pdf_dir_w = bsdf.pdf(is.out_dir, photon_in_dir);
-        const float pdf_rev_w = bsdf.pdf(photon_in_dir, is.out_dir);
-        if (pdf_dir_w == 0.0f || pdf_rev_w == 0.0f || is_black(bsdf_value)) continue;
-        const float mis_weight_light = q3.w * p.eta_vc + q4.w * pdf_dir_w;
-        const float mis_weight_camera = dVCM * p.eta_vc + dVM * pdf_rev_w;
-        const float mis_weight = p.algo == kAlgoPpm ? 1.0f : (1.0f / (mis_weight_light + 1.0f + mis_weight_camera));
-        const V3 dp = v3(q0) - is.pos;
-        const float d = dot(dp, dp);
-        const float kernel = 1.0f - d / radius_sqr;
-        contrib = contrib + mis_weight * bsdf_value * kernel * v3(q6);
-    }
-    contrib = contrib * (2.0f / (kPi * radius_sqr * (float)p.light_path_count));
-    return thr * contrib;
-}
-
 // A camera vertex waiting for merging (7 float4): pos + pixel, out_dir + material, normal +
 // dVCM, geometric normal + dVM, u tangent + uv.x, v tangent + uv.y, throughput.
 constexpr int kMergeRec = 7;
 
-// Vertex merging for the camera vertices queued by the shading kernel (count on the device).
-__global__ void __launch_bounds__(128) vcm_merge_kernel(VcmParams p, const int* count, const float4* recs) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= *count) return;
-    const float4* r = recs + kMergeRec * (size_t)i;
-    const float4 m0 = r[0], m1 = r[1], m2 = r[2], m3 = r[3], m4 = r[4], m5 = r[5], m6 = r[6];
-    Isect is;
-    is.pos = v3(m0);
-    is.out_dir = v3(m1);
-    is.normal = v3(m2);
-    is.geom_normal = v3(m3);
-    is.u_tangent = v3(m4);
-    is.v_tangent = v3(m5);
-    is.mat = __float_as_int(m1.w);
-    const Bsdf bsdf = surface_bsdf(p.s, p.s.materials[is.mat], is.normal, is.u_tangent, is.v_tangent, is.geom_normal,
-                                   m4.w, m5.w, false);
-    add_image(p.image, __float_as_int(m0.w), vcm_merge(p, v3(m6), m2.w, m3.w, is, bsdf));
-}
-
-// Vertex merging with one warp per queued camera vertex (k <= 32): the warp's k-nearest
-// search (grid_query_knn_warp, one list entry per lane), the found photons evaluated one per
-// lane, and their contributions summed in list order, so the result equals the per-thread
-// query's.
-__global__ void __launch_bounds__(128) vcm_merge_warp_kernel(VcmParams p, const int* count_ptr, const float4* recs) {
+// VCMIntegrator::vertex_merging (vcm.cpp:571-611) for the camera vertices queued by the shading
+// kernel (count on the device), one warp per vertex: the warp's k-nearest search
+// (grid_query_knn_warp), the found photons evaluated one per lane, and their contributions
+// summed in list order as the reference accumulates them.
+template <int kCap>
+__global__ void __launch_bounds__(128, 8) vcm_merge_warp_kernel(VcmParams p, const int* count_ptr, const float4* recs) {
+    __shared__ float prm[10];
+    __shared__ KnnScratch<kCap> scratch[4];
+    if (threadIdx.x < 10) prm[threadIdx.x] = __ldg(p.grid_params + threadIdx.x);
+    __syncthreads();
     const int lane = threadIdx.x & 31;
     const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (q >= *count_ptr) return;   // uniform across the warp
     const float4* r = recs + kMergeRec * (size_t)q;
-    const float4 m0 = r[0], m1 = r[1], m2 = r[2], m3 = r[3], m4 = r[4], m5 = r[5], m6 = r[6];
-    const float qx = m0.x, qy = m0.y, qz = m0.z;
-    float prm[10];
-#pragma unroll
-    for (int k = 0; k < 10; ++k) prm[k] = __ldg(p.grid_params + k);
+    const float4 m0 = r[0];
     const int k = p.num_knn;
-    float my_d;               // list entry `lane`
-    int my_id;
-    const int count = grid_query_knn_warp(p.grid_sorted, p.grid_ends, prm, p.grid_table, qx, qy, qz, k, my_d, my_id);
+    KnnScratch<kCap>& s = scratch[threadIdx.x >> 5];
+    const int count = grid_query_knn_warp<kCap>(p.grid_sorted, p.grid_ends, prm, p.grid_table, m0.x, m0.y, m0.z, k, s);
     if (count == 0) return;
-    // Evaluate the found photons, one per lane.
-    const V3 pos(qx, qy, qz), out_dir = v3(m1), thr = v3(m6);
+    const float4 m1 = r[1], m2 = r[2], m3 = r[3], m4 = r[4], m5 = r[5], m6 = r[6];
+    const V3 pos = v3(m0), out_dir = v3(m1), thr = v3(m6);
     const float dVCM = m2.w, dVM = m3.w;
     float radius_sqr = p.pm_radius * p.pm_radius;
-    V3 c(0.0f);
-    float4 lq0 = make_float4(0, 0, 0, 0);
-    if (lane < count) lq0 = __ldg(p.cache + 7 * (size_t)my_id);
     if (count == k) {
-        const V3 d = V3(__shfl_sync(0xffffffffu, lq0.x, k - 1), __shfl_sync(0xffffffffu, lq0.y, k - 1),
-                        __shfl_sync(0xffffffffu, lq0.z, k - 1)) - pos;
+        const V3 d = v3(__ldg(p.cache + 7 * (size_t)s.id[k - 1])) - pos;
         radius_sqr = dot(d, d);
     }
-    if (lane < count) {
-        const Material& mat = p.s.materials[__float_as_int(m1.w)];
-        const Bsdf bsdf = surface_bsdf(p.s, mat, v3(m2), v3(m4), v3(m5), v3(m3), m4.w, m5.w, false);
-        const float4* v = p.cache + 7 * (size_t)my_id;
-        const float4 q1 = __ldg(v + 1), q3 = __ldg(v + 3), q4 = __ldg(v + 4), q6 = __ldg(v + 6);
-        const V3 photon_in_dir = v3(q1);
-        const V3 bsdf_value = bsdf.eval(out_dir, photon_in_dir);
-        const float pdf_dir_w = bsdf.pdf(out_dir, photon_in_dir);
-        const float pdf_rev_w = bsdf.pdf(photon_in_dir, out_dir);
-        if (!(pdf_dir_w == 0.0f || pdf_rev_w == 0.0f || is_black(bsdf_value))) {
-            const float mis_weight_light = q3.w * p.eta_vc + q4.w * pdf_dir_w;
-            const float mis_weight_camera = dVCM * p.eta_vc + dVM * pdf_rev_w;
-            const float mis_weight = p.algo == kAlgoPpm ? 1.0f : (1.0f / (mis_weight_light + 1.0f + mis_weight_camera));
-            const V3 dp = v3(lq0) - pos;
-            const float d = dot(dp, dp);
-            const float kernel = 1.0f - d / radius_sqr;
-            c = mis_weight * bsdf_value * kernel * v3(q6);
-        }
-    }
-    // Sum in list order, as the reference accumulates.
     V3 contrib(0.0f);
-    for (int l = 0; l < count; ++l)
-        contrib = contrib + V3(__shfl_sync(0xffffffffu, c.x, l), __shfl_sync(0xffffffffu, c.y, l),
-                               __shfl_sync(0xffffffffu, c.z, l));
+    for (int base = 0; base < count; base += 32) {
+        V3 c(0.0f);
+        if (base + lane < count) {
+            const Material& mat = p.s.materials[__float_as_int(m1.w)];
+            const Bsdf bsdf = surface_bsdf(p.s, mat, v3(m2), v3(m4), v3(m5), v3(m3), m4.w, m5.w, false);
+            const float4* v = p.cache + 7 * (size_t)s.id[base + lane];
+            const float4 q0 = __ldg(v), q1 = __ldg(v + 1), q3 = __ldg(v + 3), q4 = __ldg(v + 4), q6 = __ldg(v + 6);
+            const V3 photon_in_dir = v3(q1);
+            const V3 bsdf_value = bsdf.eval(out_dir, photon_in_dir);
+            const float pdf_dir_w = bsdf.pdf(out_dir, photon_in_dir);
+            const float pdf_rev_w = bsdf.pdf(photon_in_dir, out_dir);
+            if (!(pdf_dir_w == 0.0f || pdf_rev_w == 0.0f || is_black(bsdf_value))) {
+                const float mis_weight_light = q3.w * p.eta_vc + q4.w * pdf_dir_w;
+                const float mis_weight_camera = dVCM * p.eta_vc + dVM * pdf_rev_w;
+                const float mis_weight =
+                    p.algo == kAlgoPpm ? 1.0f : (1.0f / (mis_weight_light + 1.0f + mis_weight_camera));
+                const V3 dp = v3(q0) - pos;
+                const float d = dot(dp, dp);
+                const float kernel = 1.0f - d / radius_sqr;
+                c = mis_weight * bsdf_value * kernel * v3(q6);
+            }
+        }
+        const int m = min(count - base, 32);
+        for (int l = 0; l < m; ++l)
+            contrib = contrib + V3(__shfl_sync(0xffffffffu, c.x, l), __shfl_sync(0xffffffffu, c.y, l),
+                                   __shfl_sync(0xffffffffu, c.z, l));
+    }
     if (lane == 0) {
         contrib = contrib * (2.0f / (kPi * radius_sqr * (float)p.light_path_count));
         add_image(p.image, __float_as_int(m0.w), thr * contrib);
@@ -737,7 +680,7 @@ __global__ void __launch_bounds__(128) vcm_camera_shade_kernel(
             }
         }
     }
-    // Vertex merging runs in vcm_merge_kernel over the queued camera vertices.
+    // Vertex merging runs in vcm_merge_warp_kernel over the queued camera vertices.
     const bool merge = surface && p.algo != kAlgoBpt && p.algo != kAlgoPt && nonspec && p.merging;
     const int mslot = warp_append(p.counts + 3, merge);
     if (merge) {
@@ -1395,11 +1338,9 @@ int imbart_vcm_camera_pass_range(imbart_vcm* v, const imbart_scene* scene, const
                 v->s_contrib, v->c_merge, v->use_perm ? v->perm : nullptr);
             note_launches(1);
             if (p.merging && (st->algorithm == IMBART_VCM || st->algorithm == IMBART_PPM)) {
-                if (st->num_knn <= 32)   // one warp per queued vertex
-                    vcm_merge_warp_kernel<<<(int)(((long long)n * 32 + 127) / 128), 128, 0, s>>>(p, v->counts + 3,
-                                                                                               v->c_merge);
-                else
-                    vcm_merge_kernel<<<(n + 127) / 128, 128, 0, s>>>(p, v->counts + 3, v->c_merge);
+                const auto merge = st->num_knn <= 32 ? vcm_merge_warp_kernel<kKnnCapSmall>
+                                                     : vcm_merge_warp_kernel<kKnnCapLarge>;
+                merge<<<(int)(((long long)n * 32 + 127) / 128), 128, 0, s>>>(p, v->counts + 3, v->c_merge);
                 note_launches(1);
             }
             const int bound = n * per;
