@@ -152,9 +152,11 @@ void scene_pool_view_destroy(imbart_scene* s);
 void scene_pool_view_set_root(imbart_scene* s, int root, int direct_root = -1, int direct_inst = -1);
 
 // A scene over device arrays built on the GPU; the scene takes ownership (cudaFree on
-// destroy). NULL on error (the arrays are then still the caller's).
+// destroy). NULL on error (the arrays are then still the caller's). direct_root / direct_inst:
+// mesh root and id of a top level that is one identity instance (-1: none).
 imbart_scene* scene_adopt_device_arrays(int device, WideNode* nodes, int64_t n_nodes, int64_t top_nodes,
-                                        WideTri* tris, int64_t n_tris, WideInst* insts, int64_t n_insts, int root);
+                                        WideTri* tris, int64_t n_tris, WideInst* insts, int64_t n_insts, int root,
+                                        int direct_root, int direct_inst);
 
 // imbart_estimate_pixel_size with the scratch buffers of a VCM context (kept between calls,
 // so that repeated estimates allocate nothing once the context has grown to the image size).

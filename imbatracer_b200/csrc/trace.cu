@@ -529,8 +529,11 @@ void scene_pool_view_set_root(imbart_scene* s, int root, int direct_root, int di
 }
 
 imbart_scene* scene_adopt_device_arrays(int device, WideNode* nodes, int64_t n_nodes, int64_t top_nodes,
-                                        WideTri* tris, int64_t n_tris, WideInst* insts, int64_t n_insts, int root) {
+                                        WideTri* tris, int64_t n_tris, WideInst* insts, int64_t n_insts, int root,
+                                        int direct_root, int direct_inst) {
     imbart_scene* s = new imbart_scene;
+    s->direct_root = direct_root;
+    s->direct_inst = direct_inst;
     s->device = device;
     s->nodes = nodes;
     s->tris = tris;

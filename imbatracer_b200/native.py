@@ -91,6 +91,10 @@ class InstanceDesc(C.Structure):
                 ("id", C.c_int)]
 
 
+INSTANCE_DESC_DTYPE = np.dtype([("obj_to_world", "<f4", 12), ("world_to_obj", "<f4", 12), ("mesh", "<i4"), ("id", "<i4")])
+assert C.sizeof(InstanceDesc) == INSTANCE_DESC_DTYPE.itemsize
+
+
 class VcmRequest(C.Structure):
     _fields_ = [("scene", C.c_int), ("camera", Camera), ("settings", VcmSettings), ("radius_factor", C.c_float),
                 ("iterations", C.c_int), ("seed_step", C.c_ulonglong), ("image_host", C.c_void_p)]

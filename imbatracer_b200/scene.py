@@ -256,11 +256,12 @@ def build_descs(meshes: list[Mesh], instances: list[Instance]):
         md[k].tri_offset = off
         off += m.triangle_count
     idesc = (N.InstanceDesc * len(instances))()
-    for i, inst in enumerate(instances):
-        idesc[i].obj_to_world[:] = [float(x) for x in inst.mat[:3].reshape(-1)]
-        idesc[i].world_to_obj[:] = [float(x) for x in inst.inv_mat.reshape(-1)]
-        idesc[i].mesh = inst.mesh_id
-        idesc[i].id = i
+    if instances:
+        rows = np.frombuffer(idesc, N.INSTANCE_DESC_DTYPE)     # the descriptors' own memory
+        rows["obj_to_world"] = [inst.mat[:3].reshape(-1) for inst in instances]
+        rows["world_to_obj"] = [inst.inv_mat.reshape(-1) for inst in instances]
+        rows["mesh"] = [inst.mesh_id for inst in instances]
+        rows["id"] = np.arange(len(instances))
     return md, idesc, keep
 
 

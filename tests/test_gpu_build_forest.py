@@ -1,0 +1,82 @@
+"""The device builder builds all meshes' trees and the instances' tree as one forest: meshes from
+one triangle up, many more trees than a block has threads, sizes at the edges of a block's tile
+and of the clusters one block finishes alone, and coinciding triangles (equal keys, no extent)."""
+import numpy as np
+import pytest
+
+from imbatracer_b200 import scene as S
+from imbatracer_b200 import scenegen as G
+from oracle import oracle as O
+from tests import helpers as H
+from tests.test_gpu_build import _DeviceBytes, trace
+
+
+def soup(rng, n, extent=6.0, size=0.7):
+    c = rng.uniform(-extent, extent, (n, 1, 3))
+    v = (c + rng.normal(scale=size, size=(n, 3, 3))).reshape(-1, 3)
+    idx = np.concatenate([np.arange(3 * n).reshape(n, 3), np.zeros((n, 1), int)], 1)
+    return S.Mesh(v.astype(np.float32), idx.astype(np.int32))
+
+
+def placed(rng, mesh):
+    m = np.eye(4)
+    m[:3, :3] = G.rotation(rng) * rng.uniform(0.4, 1.5)
+    m[:3, 3] = rng.uniform(-8, 8, 3)
+    return S.Instance(mesh, m.astype(np.float32))
+
+
+def forest(name):
+    rng = np.random.default_rng(17)
+    if name == "one":
+        return [soup(rng, 1)], [S.Instance(0)]
+    if name == "tiny trees":
+        meshes = [soup(rng, int(n), 1.0, 1.0) for n in rng.integers(1, 5, 700)]
+        return meshes, [placed(rng, i % 700) for i in range(900)]
+    if name == "edges":
+        meshes = [soup(rng, n) for n in (2, 3, 4, 31, 255, 256, 257, 2047, 2048, 2049, 4500)]
+        return meshes, [placed(rng, i) for i in range(len(meshes))]
+    if name == "coinciding":
+        m = soup(rng, 1, 0.0, 3.0)
+        v = np.tile(m.vertices, (1500, 1))
+        idx = np.concatenate([np.arange(4500).reshape(1500, 3), np.zeros((1500, 1), int)], 1).astype(np.int32)
+        return [S.Mesh(v, idx), soup(rng, 40)], [S.Instance(0), S.Instance(1)]
+    return [soup(rng, 70000, 10.0, 0.1)], [S.Instance(0)]      # "large": several blocks, one tree
+
+
+def records(ds, which, count, size):
+    import torch
+    raw = torch.as_tensor(_DeviceBytes(ds.device_arrays()[which], count * size), device="cuda").cpu().numpy()
+    return raw.reshape(count, size)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["one", "tiny trees", "edges", "coinciding", "large"])
+def test_forest_build_and_refit(cuda, name):
+    meshes, instances = forest(name)
+    n_tris = sum(m.triangle_count for m in meshes)
+    ds = S.DeviceScene.build_gpu(meshes, instances)
+    assert ds.info.triangles == n_tris and ds.info.instances == len(instances)
+    ids = records(ds, 1, n_tris, 48)[:, 12:16].copy().view(np.int32)[:, 0]
+    assert np.array_equal(np.sort(ids), np.arange(n_tris))                 # every triangle in one leaf
+    nodes = records(ds, 0, int(ds.info.wide_nodes), 80)
+    bottom = int(ds.info.wide_nodes - ds.info.top_nodes)
+    counts = nodes[:, 24:32] >> 5
+    assert counts[:bottom].sum() == n_tris and counts[bottom:].sum() == len(instances)
+    assert counts.max() <= 3 and counts[bottom:].max() == 1
+    internal = np.unpackbits(nodes[:, 15]).sum()
+    assert internal == len(nodes) - len(meshes) - 1                        # every node but the roots has a parent
+    layout = np.concatenate([[0], np.cumsum([m.triangle_count for m in meshes])[:-1]]).astype(np.int32)
+    rays = G.random_rays(np.random.default_rng(3), 1500, [-9] * 3, [9] * 3)
+    want = O.trace_brute(meshes, instances, layout, rays)
+    got, _ = trace(ds, rays)
+    assert (want["tri_id"] >= 0).any() or name == "one"
+    assert H.hits_equal(want, got).all()
+    # Moved twice: the second refit finds the counters the first one left.
+    for step in (1, 2):
+        moved = [S.Mesh((m.vertices * np.float32(1 + 0.1 * step)), m.indices, m.normals, m.texcoords, m.geom_normals)
+                 for m in meshes]
+        ds.refit(moved)
+        want = O.trace_brute(moved, instances, layout, rays)
+        got, _ = trace(ds, rays)
+        assert H.hits_equal(want, got).all()
+    ds.close()
