@@ -537,48 +537,34 @@ __device__ __forceinline__ void quantize_axis_octet(float lo, float hi, bool val
     bexp_out = e + 127;
 }
 
-// The same for a serial caller with all eight boxes (refit).
-__device__ void quantize_axis_dev(const float* lo, const float* hi, const bool* valid, float pad, float* p_out,
-                                  uint8_t* bexp_out, uint8_t* qlo, uint8_t* qhi) {
-    double nlo = DBL_MAX, nhi = -DBL_MAX;
-    for (int i = 0; i < 8; ++i) {
-        if (!valid[i]) continue;
-        nlo = fmin(nlo, (double)lo[i] - pad);
-        nhi = fmax(nhi, (double)hi[i] + pad);
-    }
-    if (nlo > nhi) { nlo = 0.0; nhi = 0.0; }
-    const double ext = nhi - nlo;
-    int e = -126;
-    if (ext > 0.0) {
-        int ex;
-        frexp(ext / 252.0, &ex);
-        e = max(ex - 1, -126);
-        while (e < 127 && ldexp(252.0, e) < ext) ++e;
-    }
-    float P = 0.0f;
-    for (;;) {
-        const double s = ldexp(1.0, e);
-        const double margin = s / 128.0;
-        const double origin = nlo - margin - 32768.0 * s;
-        P = (float)origin;
-        if ((double)P > origin) P = nextafterf(P, -FLT_MAX);
-        bool ok = true;
-        for (int i = 0; i < 8; ++i) {
-            if (!valid[i]) { qlo[i] = 1; qhi[i] = 0; continue; }
-            const double L = (double)lo[i] - pad - margin, H = (double)hi[i] + pad + margin;
-            double ql = floor((L - (double)P) / s) - 32768.0;
-            double qh = ceil((H - (double)P) / s) - 32768.0;
-            for (int g = 0; g < 64 && (double)P + (32768.0 + ql) * s > L; ++g) ql -= 1;
-            for (int g = 0; g < 64 && (double)P + (32768.0 + qh) * s < H; ++g) qh += 1;
-            if (!(ql >= 0 && qh <= 255)) { ok = false; break; }
-            qlo[i] = (uint8_t)ql;
-            qhi[i] = (uint8_t)qh;
+// The child boxes of one node (lane s: slot s, zero where not valid) padded and quantized into
+// its byte planes, words 8 to 19 of the record w (written if active); returns origin and exponents.
+__device__ __forceinline__ void quantize_octet(bool active, const Box6& b, bool valid, uint32_t* w, float p[3],
+                                               int bexp[3]) {
+    const unsigned full = 0xffffffffu;
+    const int lane8 = threadIdx.x & 7;
+    float mag = 0.0f;
+    if (valid)
+        for (int a = 0; a < 3; ++a) {
+            mag = fmaxf(mag, fmaxf(fabsf(b.lo[a]), fabsf(b.hi[a])));
+            mag = fmaxf(mag, b.hi[a] - b.lo[a]);
         }
-        if (ok || e >= 127) break;
-        ++e;
+    for (int o = 4; o > 0; o >>= 1) mag = fmaxf(mag, __shfl_xor_sync(full, mag, o));
+    const float pad = mag * 9.5367431640625e-07f + 1e-30f;
+    // Lanes 0-3 make the first word of each byte row, lanes 4-7 the second.
+    const int half = lane8 >> 2;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        uint32_t ql, qh;
+        quantize_axis_octet(b.lo[a], b.hi[a], valid, pad, p[a], bexp[a], ql, qh);
+        ql <<= 8 * (lane8 & 3);
+        qh <<= 8 * (lane8 & 3);
+        for (int o = 2; o > 0; o >>= 1) {
+            ql |= __shfl_xor_sync(full, ql, o);
+            qh |= __shfl_xor_sync(full, qh, o);
+        }
+        if (active && (lane8 & 3) == 0) { w[8 + 4 * a + half] = ql; w[10 + 4 * a + half] = qh; }
     }
-    *p_out = P;
-    *bexp_out = (uint8_t)(e + 127);
 }
 
 // Where the leaves' records go.
@@ -749,34 +735,13 @@ __device__ __forceinline__ void write_wide(const Forest& f, bool active, int kid
             }
         }
     }
-    float mag = 0.0f;
-    if (valid)
-        for (int a = 0; a < 3; ++a) {
-            mag = fmaxf(mag, fmaxf(fabsf(b.lo[a]), fabsf(b.hi[a])));
-            mag = fmaxf(mag, b.hi[a] - b.lo[a]);
-        }
-    for (int o = 4; o > 0; o >>= 1) mag = fmaxf(mag, __shfl_xor_sync(full, mag, o));
-    const float pad = mag * 9.5367431640625e-07f + 1e-30f;
-    float p[3];
-    int bexp[3];
     uint32_t* w = reinterpret_cast<uint32_t*>(out);
-    const int half = lane8 >> 2;          // lanes 0-3 make the first word of each byte row, 4-7 the second
-    const bool writes = active && (lane8 & 3) == 0;
     uint32_t meta = (uint32_t)((count << 5) | (count > 0 ? poff : 0)) << (8 * (lane8 & 3));
     for (int o = 2; o > 0; o >>= 1) meta |= __shfl_xor_sync(full, meta, o);
-    if (writes) w[6 + half] = meta;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        uint32_t ql, qh;
-        quantize_axis_octet(b.lo[a], b.hi[a], valid, pad, p[a], bexp[a], ql, qh);
-        ql <<= 8 * (lane8 & 3);
-        qh <<= 8 * (lane8 & 3);
-        for (int o = 2; o > 0; o >>= 1) {
-            ql |= __shfl_xor_sync(full, ql, o);
-            qh |= __shfl_xor_sync(full, qh, o);
-        }
-        if (writes) { w[8 + 4 * a + half] = ql; w[10 + 4 * a + half] = qh; }
-    }
+    if (active && (lane8 & 3) == 0) w[6 + (lane8 >> 2)] = meta;
+    float p[3];
+    int bexp[3];
+    quantize_octet(active, b, valid, w, p, bexp);
     if (active && lane8 == 0) {
         w[0] = __float_as_uint(p[0]);
         w[1] = __float_as_uint(p[1]);
@@ -1168,32 +1133,18 @@ int build_scene_gpu(const imbart_mesh_desc* meshes, int n_meshes, const imbart_i
 // Refit: the vertices moved, the topology did not. Triangle records take their triangle's
 // new vertices; node boxes are recomputed bottom-up (bottom levels, then the instances'
 // world boxes, then the top level) and requantized with the build's conservative
-// arithmetic. Each leaf-only node starts a thread that refits it and climbs: the last child
-// of a parent to finish refits the parent (a counter per node).
+// arithmetic. Eight lanes start at each node without internal children, a lane per slot, and
+// climb: the last child of a parent to finish refits the parent (a counter per node, back at
+// its start value afterwards, so that it serves every refit of the scene). The chain of a leaf's
+// ancestors bounds a refit, hence eight lanes for a node's children, boxes and bytes. Measured
+// (B200), 512 k triangles, with 65,536 rays traced after it: 960 us with a thread per node and
+// scratch allocated by every refit, 276 us.
 // ---------------------------------------------------------------------------------------
-__global__ void refit_tris_kernel(WideTri* tris, long long n, const float* __restrict__ verts,
-                                  const int4* __restrict__ tri_verts, int n_tri_ids, long long n_verts, int* error) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    WideTri t = tris[i];
-    if (t.id < 0 || t.id >= n_tri_ids) { atomicExch(error, 1); return; }
-    const int4 v = tri_verts[t.id];
-    if (v.x < 0 || v.y < 0 || v.z < 0 || v.x >= n_verts || v.y >= n_verts || v.z >= n_verts) {
-        atomicExch(error, 2);
-        return;
-    }
-    for (int k = 0; k < 3; ++k) {
-        t.v0[k] = verts[3 * (long long)v.x + k];
-        t.v1[k] = verts[3 * (long long)v.y + k];
-        t.v2[k] = verts[3 * (long long)v.z + k];
-    }
-    tris[i] = t;
-}
 
-// Parent of every internal child and the count of internal children of nodes [first, last).
-__global__ void refit_links_kernel(const WideNode* __restrict__ nodes, int first, int last, int* parent, int* pending) {
-    const int n = first + blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= last) return;
+// Parent of every internal child (-1: none) and the count of internal children of each node.
+__global__ void refit_links_kernel(const WideNode* __restrict__ nodes, int n_nodes, int* parent, int* pending) {
+    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= n_nodes) return;
     const WideNode nd = nodes[n];
     pending[n] = __popc(nd.imask);
     int rank = 0;
@@ -1215,69 +1166,108 @@ __device__ __forceinline__ Box6 load_box_cg(const Box6* p) {
     return b;
 }
 
-// Requantizes node n from its children (leaf slots: their triangles or instances; internal
-// slots: the boxes their refits stored) and stores its own box.
-__device__ void refit_node(WideNode* nodes, int n, const WideTri* __restrict__ tris, const Box6* inst_boxes, bool top,
-                           Box6* exact) {
-    WideNode nd = nodes[n];
-    float blo[3][8], bhi[3][8];
-    bool valid[8];
-    float mag = 0.0f;
-    Box6 all = empty_box();
-    int rank = 0;
-    for (int s = 0; s < 8; ++s) {
-        Box6 b = empty_box();
-        if (nd.imask & (1u << s)) {
-            b = load_box_cg(exact + nd.child_base + rank++);
-            valid[s] = true;
+// The moved vertices of a bottom-level refit.
+struct MovedVerts {
+    const float* verts;
+    long long n_verts;
+    const int4* tri_verts;
+    int n_tri_ids;
+    int* error;
+};
+
+// Moves triangle record t to its new vertices and returns its box; a bad id or index sets
+// *error and leaves the record.
+__device__ __forceinline__ Box6 move_triangle(WideTri* t, const MovedVerts& m) {
+    float4* r = reinterpret_cast<float4*>(t);
+    float4 v0 = r[0], v1 = r[1], v2 = r[2];
+    const int id = __float_as_int(v0.w);
+    if (id < 0 || id >= m.n_tri_ids) {
+        atomicExch(m.error, 1);
+    } else {
+        const int4 i = __ldg(m.tri_verts + id);
+        if (i.x < 0 || i.y < 0 || i.z < 0 || i.x >= m.n_verts || i.y >= m.n_verts || i.z >= m.n_verts) {
+            atomicExch(m.error, 2);
         } else {
-            const int count = nd.meta[s] >> 5, off = nd.meta[s] & 31;
-            valid[s] = count > 0;
-            for (int k = 0; k < count; ++k) {
-                const long long r = (long long)nd.prim_base + off + k;
-                if (top) {
-                    b = merge(b, inst_boxes[r]);
-                } else {
-                    const WideTri t = tris[r];
-                    for (int a = 0; a < 3; ++a) {
-                        b.lo[a] = fminf(b.lo[a], fminf(t.v0[a], fminf(t.v1[a], t.v2[a])));
-                        b.hi[a] = fmaxf(b.hi[a], fmaxf(t.v0[a], fmaxf(t.v1[a], t.v2[a])));
-                    }
-                }
-            }
-        }
-        for (int a = 0; a < 3; ++a) { blo[a][s] = valid[s] ? b.lo[a] : 0.0f; bhi[a][s] = valid[s] ? b.hi[a] : 0.0f; }
-        if (!valid[s]) continue;
-        all = merge(all, b);
-        for (int a = 0; a < 3; ++a) {
-            mag = fmaxf(mag, fmaxf(fabsf(b.lo[a]), fabsf(b.hi[a])));
-            mag = fmaxf(mag, b.hi[a] - b.lo[a]);
+            const float *a = m.verts + 3ll * i.x, *b = m.verts + 3ll * i.y, *c = m.verts + 3ll * i.z;
+            v0.x = __ldg(a); v0.y = __ldg(a + 1); v0.z = __ldg(a + 2);
+            v1.x = __ldg(b); v1.y = __ldg(b + 1); v1.z = __ldg(b + 2);
+            v2.x = __ldg(c); v2.y = __ldg(c + 1); v2.z = __ldg(c + 2);
+            r[0] = v0; r[1] = v1; r[2] = v2;
         }
     }
-    const float pad = mag * 9.5367431640625e-07f + 1e-30f;
-    float p[3];
-    uint8_t bexp[3];
-    quantize_axis_dev(blo[0], bhi[0], valid, pad, &p[0], &bexp[0], nd.qlo_x, nd.qhi_x);
-    quantize_axis_dev(blo[1], bhi[1], valid, pad, &p[1], &bexp[1], nd.qlo_y, nd.qhi_y);
-    quantize_axis_dev(blo[2], bhi[2], valid, pad, &p[2], &bexp[2], nd.qlo_z, nd.qhi_z);
-    nd.px = p[0]; nd.py = p[1]; nd.pz = p[2];
-    nd.ex = bexp[0]; nd.ey = bexp[1]; nd.ez = bexp[2];
-    nodes[n] = nd;
-    exact[n] = all;
+    Box6 x;
+    x.lo[0] = fminf(v0.x, fminf(v1.x, v2.x)); x.hi[0] = fmaxf(v0.x, fmaxf(v1.x, v2.x));
+    x.lo[1] = fminf(v0.y, fminf(v1.y, v2.y)); x.hi[1] = fmaxf(v0.y, fmaxf(v1.y, v2.y));
+    x.lo[2] = fminf(v0.z, fminf(v1.z, v2.z)); x.hi[2] = fmaxf(v0.z, fmaxf(v1.z, v2.z));
+    return x;
 }
 
-__global__ void refit_up_kernel(WideNode* nodes, int first, int last, const int* __restrict__ parent, int* pending,
-                                const WideTri* __restrict__ tris, const Box6* inst_boxes, bool top, Box6* exact) {
-    int n = first + blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= last || nodes[n].imask != 0) return;
-    for (;;) {
-        refit_node(nodes, n, tris, inst_boxes, top, exact);
-        __threadfence();
-        const int p = parent[n];
-        if (p < 0) return;
-        if (atomicSub(pending + p, 1) != 1) return;   // the parent's last child to finish goes on
-        __threadfence();
-        n = p;
+// Refits node n of an active octet: lane s takes slot s (leaf slots: their triangles, moved, or
+// instances; internal slots: the boxes their refits stored); the node's own box goes to exact.
+__device__ __forceinline__ void refit_node(bool active, WideNode* nodes, int n, WideTri* tris, const MovedVerts& mv,
+                                           const Box6* inst_boxes, Box6* exact) {
+    const unsigned full = 0xffffffffu;
+    const int lane8 = threadIdx.x & 7;
+    uint32_t* w = reinterpret_cast<uint32_t*>(nodes + n);
+    Box6 b = empty_box();
+    bool valid = false;
+    uint32_t imask = 0u;
+    if (active) {
+        imask = w[3] >> 24;
+        if ((imask >> lane8) & 1u) {
+            valid = true;
+            b = load_box_cg(exact + w[4] + __popc(imask & ((1u << lane8) - 1u)));
+        } else {
+            const uint32_t meta = (w[6 + (lane8 >> 2)] >> (8 * (lane8 & 3))) & 0xffu;
+            const int count = (int)(meta >> 5);
+            const long long first = (long long)w[5] + (meta & 31u);
+            valid = count > 0;
+            for (int k = 0; k < count; ++k)
+                b = merge(b, inst_boxes ? inst_boxes[first + k] : move_triangle(tris + first + k, mv));
+        }
+    }
+    Box6 all = b;
+    for (int o = 4; o > 0; o >>= 1)
+        for (int a = 0; a < 3; ++a) {
+            all.lo[a] = fminf(all.lo[a], __shfl_xor_sync(full, all.lo[a], o));
+            all.hi[a] = fmaxf(all.hi[a], __shfl_xor_sync(full, all.hi[a], o));
+        }
+    if (!valid)
+        for (int a = 0; a < 3; ++a) b.lo[a] = b.hi[a] = 0.0f;
+    float p[3];
+    int bexp[3];
+    quantize_octet(active, b, valid, w, p, bexp);
+    if (active && lane8 == 0) {
+        w[0] = __float_as_uint(p[0]);
+        w[1] = __float_as_uint(p[1]);
+        w[2] = __float_as_uint(p[2]);
+        w[3] = (uint32_t)bexp[0] | ((uint32_t)bexp[1] << 8) | ((uint32_t)bexp[2] << 16) | (imask << 24);
+        float* e = reinterpret_cast<float*>(exact + n);
+        for (int a = 0; a < 3; ++a) { e[a] = all.lo[a]; e[3 + a] = all.hi[a]; }
+    }
+}
+
+__global__ void __launch_bounds__(kBlock) refit_up_kernel(WideNode* nodes, int first, int last,
+                                                          const int* __restrict__ parent, int* pending, WideTri* tris,
+                                                          MovedVerts mv, const Box6* inst_boxes, Box6* exact) {
+    const unsigned full = 0xffffffffu;
+    const int lane8 = threadIdx.x & 7;
+    int n = first + (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 3);
+    bool active = n < last && nodes[n].imask == 0;
+    while (__ballot_sync(full, active) != 0u) {
+        refit_node(active, nodes, n, tris, mv, inst_boxes, exact);
+        int up = -1;
+        if (active && lane8 == 0) {
+            __threadfence();
+            const int p = parent[n];
+            if (p >= 0 && atomicSub(pending + p, 1) == 1) {   // the parent's last child to finish goes on
+                __threadfence();
+                pending[p] = __popc(nodes[p].imask);
+                up = p;
+            }
+        }
+        n = __shfl_sync(full, up, 0, 8);
+        active = n >= 0;
     }
 }
 
@@ -1343,25 +1333,40 @@ int refit_scene(imbart_scene* scene, const float* verts, long long n_verts, cons
     WideTri* tris = static_cast<WideTri*>(const_cast<void*>(vt));
     const WideInst* insts = static_cast<const WideInst*>(vi);
     const int n_nodes = (int)info.wide_nodes, first_top = (int)(info.wide_nodes - info.top_nodes);
+    // Scratch of the scene's refits, kept with the scene: parents and child counters (filled by the
+    // first refit, the topology never changes), node and instance boxes, the error word.
+    Slab slab;
     Box6 *exact = nullptr, *inst_boxes = nullptr;
     int *parent = nullptr, *pending = nullptr, *error = nullptr;
-    bool good = dmalloc(&exact, n_nodes) && dmalloc(&inst_boxes, info.instances) && dmalloc(&parent, n_nodes) &&
-                dmalloc(&pending, n_nodes) && dmalloc(&error, 1) &&
-                ck(cudaMemsetAsync(parent, 0xff, sizeof(int) * (size_t)n_nodes, st), "cudaMemsetAsync") &&
-                ck(cudaMemsetAsync(error, 0, sizeof(int), st), "cudaMemsetAsync");
+    auto layout = [&] {
+        slab.used = 0;
+        slab.take(exact, n_nodes);
+        slab.take(inst_boxes, info.instances);
+        slab.take(parent, n_nodes);
+        slab.take(pending, n_nodes);
+        slab.take(error, 1);
+    };
+    layout();
+    bool fresh = false;
+    slab.base = static_cast<char*>(scene_refit_scratch(scene, slab.used, &fresh));
+    if (!slab.base) return imbart_last_error() ? imbart_last_error() : IMBART_ERR_OUT_OF_MEMORY;
+    layout();
+    bool good = ck(cudaMemsetAsync(error, 0, sizeof(int), st), "cudaMemsetAsync");
+    if (good && fresh) {
+        good = ck(cudaMemsetAsync(parent, 0xff, sizeof(int) * (size_t)n_nodes, st), "cudaMemsetAsync");
+        if (good) refit_links_kernel<<<grid(n_nodes), kBlock, 0, st>>>(nodes, n_nodes, parent, pending);
+        note_launches(1);
+    }
     if (good) {
-        refit_tris_kernel<<<grid(info.triangles), kBlock, 0, st>>>(tris, info.triangles, verts,
-                                                                    reinterpret_cast<const int4*>(tri_verts), n_tri_ids,
-                                                                    n_verts, error);
-        refit_links_kernel<<<grid(n_nodes), kBlock, 0, st>>>(nodes, 0, n_nodes, parent, pending);
+        const MovedVerts mv{verts, n_verts, reinterpret_cast<const int4*>(tri_verts), n_tri_ids, error};
         if (first_top > 0)
-            refit_up_kernel<<<grid(first_top), kBlock, 0, st>>>(nodes, 0, first_top, parent, pending, tris, nullptr,
-                                                               false, exact);
+            refit_up_kernel<<<grid(8ll * first_top), kBlock, 0, st>>>(nodes, 0, first_top, parent, pending, tris, mv,
+                                                                     nullptr, exact);
         refit_inst_boxes_kernel<<<grid(info.instances), kBlock, 0, st>>>(insts, (int)info.instances, exact,
                                                                         inst_boxes);
-        refit_up_kernel<<<grid(info.top_nodes), kBlock, 0, st>>>(nodes, first_top, n_nodes, parent, pending, tris,
-                                                                inst_boxes, true, exact);
-        note_launches(first_top > 0 ? 5 : 4);
+        refit_up_kernel<<<grid(8ll * info.top_nodes), kBlock, 0, st>>>(nodes, first_top, n_nodes, parent, pending, tris,
+                                                                      mv, inst_boxes, exact);
+        note_launches(first_top > 0 ? 3 : 2);
         int h_error = 0;
         good = ck(cudaGetLastError(), "refit launch") &&
                ck(cudaMemcpyAsync(&h_error, error, sizeof(int), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync") &&
@@ -1372,7 +1377,7 @@ int refit_scene(imbart_scene* scene, const float* verts, long long n_verts, cons
             good = false;
         }
     }
-    cudaFree(exact); cudaFree(inst_boxes); cudaFree(parent); cudaFree(pending); cudaFree(error);
+    if (!good && fresh) scene_refit_scratch(scene, 0, &fresh);   // links may be missing: start over next time
     return good ? 0 : (imbart_last_error() ? imbart_last_error() : IMBART_ERR_CUDA);
 }
 

@@ -158,6 +158,10 @@ imbart_scene* scene_adopt_device_arrays(int device, WideNode* nodes, int64_t n_n
                                         WideTri* tris, int64_t n_tris, WideInst* insts, int64_t n_insts, int root,
                                         int direct_root, int direct_inst);
 
+// Device scratch of `bytes` for a scene's refits, allocated by the first call and freed with the
+// scene (*fresh: this call allocated it). NULL on error. bytes = 0 frees it.
+void* scene_refit_scratch(imbart_scene* s, size_t bytes, bool* fresh);
+
 // imbart_estimate_pixel_size with the scratch buffers of a VCM context (kept between calls,
 // so that repeated estimates allocate nothing once the context has grown to the image size).
 int vcm_estimate_pixel_size(imbart_vcm* v, const imbart_scene* scene, const imbart_camera* cam, float* pixel_size,

@@ -35,6 +35,7 @@ struct imbart_scene {
     float grid_share = 1.0f;   // persistent launches use this share of the resident block slots
     // Top level = one identity instance: its wide root and id (TraceParams::direct_root).
     int direct_root = -1, direct_inst = -1;
+    void* refit_scratch = nullptr;   // kept between refits (scene_refit_scratch)
     imbart_scene() { info.node_width = 8; }   // converted scenes overwrite it
 };
 
@@ -68,6 +69,7 @@ void free_scene(imbart_scene* s) {
         cudaFree(s->indices); cudaFree(s->texcoords); cudaFree(s->masks); cudaFree(s->mask_buffer);
     }
     cudaFree(s->error_flags);
+    cudaFree(s->refit_scratch);
     cudaSetDevice(prev);
     delete s;
 }
@@ -498,6 +500,16 @@ void trace_config_snapshot(int out[10]) {
     out[0] = c.variant; out[1] = c.refill; out[2] = c.postpone; out[3] = c.variant_any;
     out[4] = c.refill_any; out[5] = c.variant_coh; out[6] = c.refill_coh;
     out[7] = c.tri_batch; out[8] = c.tri_batch_any; out[9] = c.tri_batch_coh;
+}
+
+void* scene_refit_scratch(imbart_scene* s, size_t bytes, bool* fresh) {
+    if (bytes == 0) {
+        cudaFree(s->refit_scratch);
+        s->refit_scratch = nullptr;
+    }
+    *fresh = bytes > 0 && s->refit_scratch == nullptr;
+    if (*fresh && !cuda_ok(cudaMalloc(&s->refit_scratch, bytes), "cudaMalloc")) s->refit_scratch = nullptr;
+    return s->refit_scratch;
 }
 
 imbart_scene* upload_wide_scene(const HostWideScene& h, int device) { return upload_scene(h, device); }
