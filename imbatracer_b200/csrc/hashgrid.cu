@@ -10,9 +10,16 @@
 //                   axis (8 buckets in the reference's order, a bucket hit twice is scanned
 //                   twice), squared distance <= r^2, k nearest kept by insertion sort
 // Every float operation is explicitly rounded (no contraction) so that cell indices and
-// distances equal the reference's bit for bit. Within a bucket photons are placed by an
-// atomic cursor, as in the reference's parallel scatter (rangesearch.h:68-74); the query
-// returns its k photons ordered by (distance, photon index).
+// distances equal the reference's bit for bit. Within a bucket photons are placed in the order
+// an atomic counter met them, as in the reference's parallel scatter (rangesearch.h:68-74); the
+// query returns its k photons ordered by (distance, photon index).
+//
+// A build is five launches: small grids are bound by the launches and their gaps, large ones by
+// memory (the photons twice, the table three times, the sorted photons once). The bounding box's
+// and the tile sums' finishing steps run in the last block of the launch that produces them, and
+// a photon's place in its bucket is the count it got when it was counted, so the scatter needs no
+// cursors. Measured (B200): 20,011 photons with 2,000 queries 44.0 us in nine launches, 34.9 us;
+// 1.74 M photons into 2^22 buckets 80 us less.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,13 +35,13 @@ struct imbart_hashgrid {
     int device = 0;
     int n = 0;              // photons in the current build
     int table = 0;          // buckets in the current build
-    int sorted_cap = 0, cell_of_cap = 0, ends_cap = 0, cursor_cap = 0;
+    int sorted_cap = 0, place_cap = 0, ends_cap = 0;
     float4* sorted = nullptr;   // position xyz + original index (int bits) in bucket order
     int* cell_ends = nullptr;   // inclusive end of each bucket
-    int* cell_of = nullptr;     // bucket of each photon (scratch)
-    int* cursor = nullptr;      // scatter cursor per bucket (scratch)
+    int2* place = nullptr;      // bucket of each photon and its place there (scratch)
     int* block_sums = nullptr;  // scan scratch
     int block_sums_cap = 0;
+    unsigned* state = nullptr;  // 8 words, zero between builds (GridState)
     float* params = nullptr;    // device: lo[3], hi[3], radius, r^2, cell, inv_cell
     float host_params[10] = {};
     float cell_factor = 2.0f;   // cell size / radius of the current build
@@ -55,24 +62,53 @@ bool ok(cudaError_t e, const char* what) {
     return false;
 }
 
-// Order-preserving float <-> int mapping for atomicMin/atomicMax on floats.
-__device__ __forceinline__ int float_to_ordered(float f) {
-    const int i = __float_as_int(f);
-    return i >= 0 ? i : i ^ 0x7fffffff;
+// Order-preserving float -> unsigned mapping; every float maps above 0, so 0 stands for "none".
+__device__ __forceinline__ unsigned float_to_ordered(float f) {
+    const unsigned i = __float_as_uint(f);
+    return (i & 0x80000000u) ? ~i : i | 0x80000000u;
 }
-__device__ __forceinline__ float ordered_to_float(int i) {
-    return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff);
-}
-
-__global__ void bbox_init_kernel(int* box) {
-    if (threadIdx.x < 3) box[threadIdx.x] = float_to_ordered(FLT_MAX);
-    else if (threadIdx.x < 6) box[threadIdx.x] = float_to_ordered(-FLT_MAX);
+__device__ __forceinline__ float ordered_to_float(unsigned u) {
+    return __uint_as_float((u & 0x80000000u) ? u & 0x7fffffffu : ~u);
 }
 
-// Exact min/max of the positions (order-independent, so bit-identical to a serial pass).
-__global__ void bbox_kernel(const float* __restrict__ pos, int stride, int n, int* __restrict__ box) {
+// Words of a build's running state: the box as maxima (of ~ordered for the low side), then the
+// counts of finished blocks of the two launches whose last block goes on. All zero between
+// builds: the last block that reads a word clears it.
+enum GridState { kStateLo = 0, kStateHi = 3, kStateBoxDone = 6, kStateScanDone = 7, kStateWords = 8 };
+
+// True in the block of the launch that finishes last (its threads then see the other blocks'
+// writes); clears the count.
+__device__ __forceinline__ bool last_block(unsigned* done) {
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(done, 1u) == gridDim.x - 1;
+        if (last) *done = 0u;
+        __threadfence();
+    }
+    __syncthreads();
+    return last;
+}
+
+// Zeroes the bucket counts and finds the exact min / max of the positions (order-independent, so
+// bit-identical to a serial pass). The last block inflates the box (rangesearch.h:44-46) and
+// derives the cell parameters (:27-30).
+__global__ void __launch_bounds__(kBlock) bounds_kernel(const float* __restrict__ pos, int stride, int n,
+                                                        int* __restrict__ counts, int table, float radius,
+                                                        float cell_factor, float* __restrict__ prm, unsigned* state) {
+    __shared__ unsigned s_box[6];
+    const int first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    if (threadIdx.x < 6) s_box[threadIdx.x] = 0u;
+    if (((size_t)counts & 15) == 0) {
+        int4* c4 = reinterpret_cast<int4*>(counts);
+        for (int i = first; i < table / 4; i += step) c4[i] = make_int4(0, 0, 0, 0);
+        if (first < (table & 3)) counts[(table & ~3) + first] = 0;
+    } else {
+        for (int i = first; i < table; i += step) counts[i] = 0;
+    }
     float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    for (int i = first; i < n; i += step) {
         const float* p = pos + (size_t)i * stride;
         for (int a = 0; a < 3; ++a) {
             const float v = p[a];
@@ -80,36 +116,32 @@ __global__ void bbox_kernel(const float* __restrict__ pos, int stride, int n, in
             hi[a] = hi[a] > v ? hi[a] : v;
         }
     }
+    __syncthreads();
     for (int a = 0; a < 3; ++a) {
-        for (int off = 16; off > 0; off >>= 1) {
-            lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], off));
-            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], off));
-        }
+        const unsigned l = __reduce_max_sync(0xffffffffu, ~float_to_ordered(lo[a]));
+        const unsigned h = __reduce_max_sync(0xffffffffu, float_to_ordered(hi[a]));
+        if ((threadIdx.x & 31) == 0) { atomicMax(s_box + a, l); atomicMax(s_box + 3 + a, h); }
     }
-    if ((threadIdx.x & 31) == 0) {
-        for (int a = 0; a < 3; ++a) {
-            atomicMin(box + a, float_to_ordered(lo[a]));
-            atomicMax(box + 3 + a, float_to_ordered(hi[a]));
-        }
+    __syncthreads();
+    if (threadIdx.x < 6) atomicMax(state + threadIdx.x, s_box[threadIdx.x]);
+    if (!last_block(state + kStateBoxDone) || threadIdx.x != 0) return;
+    float blo[3], bhi[3], ext[3];
+    for (int a = 0; a < 3; ++a) {
+        blo[a] = ordered_to_float(~__ldcg(state + kStateLo + a));
+        bhi[a] = ordered_to_float(__ldcg(state + kStateHi + a));
+        state[kStateLo + a] = 0u;
+        state[kStateHi + a] = 0u;
     }
-}
-
-// Inflates the box (rangesearch.h:44-46) and derives the cell parameters (:27-30).
-__global__ void params_kernel(const int* __restrict__ box, float radius, float cell_factor, float* __restrict__ prm) {
-    if (threadIdx.x != 0) return;
-    float lo[3], hi[3], ext[3];
-    for (int a = 0; a < 3; ++a) { lo[a] = ordered_to_float(box[a]); hi[a] = ordered_to_float(box[3 + a]); }
-    for (int a = 0; a < 3; ++a) ext[a] = __fsub_rn(hi[a], lo[a]);
-    for (int a = 0; a < 3; ++a) hi[a] = __fadd_rn(hi[a], __fmul_rn(ext[a], 0.001f));
-    for (int a = 0; a < 3; ++a) lo[a] = __fsub_rn(lo[a], __fmul_rn(ext[a], 0.001f));
+    for (int a = 0; a < 3; ++a) ext[a] = __fsub_rn(bhi[a], blo[a]);
+    for (int a = 0; a < 3; ++a) bhi[a] = __fadd_rn(bhi[a], __fmul_rn(ext[a], 0.001f));
+    for (int a = 0; a < 3; ++a) blo[a] = __fsub_rn(blo[a], __fmul_rn(ext[a], 0.001f));
     const float cell = __fmul_rn(radius, cell_factor);
-    for (int a = 0; a < 3; ++a) { prm[a] = lo[a]; prm[3 + a] = hi[a]; }
+    for (int a = 0; a < 3; ++a) { prm[a] = blo[a]; prm[3 + a] = bhi[a]; }
     prm[6] = radius;
     prm[7] = __fmul_rn(radius, radius);
     prm[8] = cell;
     prm[9] = __fdiv_rn(1.0f, cell);
 }
-
 
 __device__ __forceinline__ int cell_of_point(const float* prm, float px, float py, float pz, uint32_t table) {
     const float inv = prm[9];
@@ -119,92 +151,104 @@ __device__ __forceinline__ int cell_of_point(const float* prm, float px, float p
     return hash_cell((uint32_t)cx, (uint32_t)cy, (uint32_t)cz, table);
 }
 
+// Counts the photons of every bucket; the count a photon gets is its place in the bucket.
 __global__ void count_kernel(const float* __restrict__ pos, int stride, int n, const float* __restrict__ prm,
-                             uint32_t table, int* __restrict__ counts, int* __restrict__ cell_of) {
+                             uint32_t table, int* __restrict__ counts, int2* __restrict__ place) {
     __shared__ float sp[10];
     if (threadIdx.x < 10) sp[threadIdx.x] = prm[threadIdx.x];
     __syncthreads();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float* p = pos + (size_t)i * stride;
         const int c = cell_of_point(sp, p[0], p[1], p[2], table);
-        cell_of[i] = c;
-        atomicAdd(counts + c, 1);
+        place[i] = make_int2(c, atomicAdd(counts + c, 1));
     }
 }
 
-// Three-phase exclusive scan: per-tile sums, scan of the tile sums, tile-local scan + offset.
-__global__ void scan_tiles_kernel(const int* __restrict__ in, int n, int* __restrict__ tile_sums) {
-    __shared__ int warp_sums[kBlock / 32];
-    const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    int s = 0;
-    for (int k = 0; k < kScanItems; ++k) s += (base + k < n) ? in[base + k] : 0;
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = 0;
-        for (int w = 0; w < kBlock / 32; ++w) t += warp_sums[w];
-        tile_sums[blockIdx.x] = t;
-    }
-}
-
-// Exclusive scan of the tile sums by one block (tiles <= kBlock * kScanItems * ... looped).
-__global__ void scan_sums_kernel(int* __restrict__ sums, int n_tiles) {
-    __shared__ int buf[kBlock];
-    int carry = 0;
-    for (int base = 0; base < n_tiles; base += kBlock) {
-        const int i = base + threadIdx.x;
-        const int v = i < n_tiles ? sums[i] : 0;
-        buf[threadIdx.x] = v;
-        __syncthreads();
-        for (int off = 1; off < kBlock; off <<= 1) {
-            const int t = threadIdx.x >= off ? buf[threadIdx.x - off] : 0;
-            __syncthreads();
-            buf[threadIdx.x] += t;
-            __syncthreads();
+// A thread's kScanItems consecutive counts, as 16-byte loads where the array allows it.
+__device__ __forceinline__ void load_items(const int* in, int base, int n, int v[kScanItems]) {
+    if (base + kScanItems <= n && ((size_t)in & 15) == 0) {
+        for (int k = 0; k < kScanItems; k += 4) {
+            const int4 q = *reinterpret_cast<const int4*>(in + base + k);
+            v[k] = q.x; v[k + 1] = q.y; v[k + 2] = q.z; v[k + 3] = q.w;
         }
-        if (i < n_tiles) sums[i] = carry + buf[threadIdx.x] - v;
-        __syncthreads();
-        carry += buf[kBlock - 1];
-        __syncthreads();
+    } else {
+        for (int k = 0; k < kScanItems; ++k) v[k] = base + k < n ? in[base + k] : 0;
     }
 }
 
-// Writes inclusive ends (cell_ends) and exclusive starts (cursor) of every bucket. `starts`
-// may alias `counts_in`: every thread reads its items before writing them.
-__global__ void scan_apply_kernel(const int* counts_in, int n, const int* __restrict__ tile_off,
-                                  int* __restrict__ ends, int* starts) {
+// Inclusive scan of one value per thread over the block (kBlock threads).
+__device__ __forceinline__ int block_scan(int v) {
     __shared__ int warp_sums[kBlock / 32];
-    const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    int v[kScanItems];
-    int s = 0;
-    for (int k = 0; k < kScanItems; ++k) { v[k] = (base + k < n) ? counts_in[base + k] : 0; s += v[k]; }
-    // exclusive scan of per-thread sums within the block
-    int incl = s;
+    int incl = v;
     for (int off = 1; off < 32; off <<= 1) {
         const int t = __shfl_up_sync(0xffffffffu, incl, off);
         if ((int)(threadIdx.x & 31) >= off) incl += t;
     }
+    __syncthreads();
     if ((threadIdx.x & 31) == 31) warp_sums[threadIdx.x >> 5] = incl;
     __syncthreads();
-    int warp_off = 0;
-    for (int w = 0; w < (int)(threadIdx.x >> 5); ++w) warp_off += warp_sums[w];
-    int run = tile_off[blockIdx.x] + warp_off + incl - s;
-    for (int k = 0; k < kScanItems; ++k) {
-        if (base + k < n) {
-            starts[base + k] = run;
-            run += v[k];
-            ends[base + k] = run;
+    for (int w = 0; w < (int)(threadIdx.x >> 5); ++w) incl += warp_sums[w];
+    return incl;
+}
+
+// Sums of the tiles of kScanTile counts; the last block turns them into exclusive offsets.
+__global__ void __launch_bounds__(kBlock) scan_tiles_kernel(const int* __restrict__ in, int n, int* tile_sums,
+                                                            unsigned* state) {
+    __shared__ int carry;
+    int v[kScanItems], s = 0;
+    load_items(in, blockIdx.x * kScanTile + threadIdx.x * kScanItems, n, v);
+    for (int k = 0; k < kScanItems; ++k) s += v[k];
+    s = block_scan(s);
+    if (threadIdx.x == kBlock - 1) tile_sums[blockIdx.x] = s;
+    if (!last_block(state + kStateScanDone)) return;
+    const int n_tiles = gridDim.x;
+    if (threadIdx.x == 0) carry = 0;
+    __syncthreads();
+    for (int base = 0; base < n_tiles; base += kScanTile) {
+        const int first = base + threadIdx.x * kScanItems;
+        int sum = 0;
+        for (int k = 0; k < kScanItems; ++k) {
+            v[k] = first + k < n_tiles ? __ldcg(tile_sums + first + k) : 0;
+            sum += v[k];
         }
+        const int incl = block_scan(sum);
+        int run = carry + incl - sum;
+        for (int k = 0; k < kScanItems; ++k) {
+            if (first + k < n_tiles) tile_sums[first + k] = run;
+            run += v[k];
+        }
+        __syncthreads();
+        if (threadIdx.x == kBlock - 1) carry = run;
+        __syncthreads();
     }
 }
 
-__global__ void scatter_kernel(const float* __restrict__ pos, int stride, int n, const int* __restrict__ cell_of,
-                               int* __restrict__ cursor, float4* __restrict__ sorted) {
+// Turns the counts into the buckets' inclusive ends, in place. Also clears the state words, so
+// that builds which overlapped on one grid (an error of the caller's) cannot spoil later ones.
+__global__ void __launch_bounds__(kBlock) scan_apply_kernel(int* ends, int n, const int* __restrict__ tile_off,
+                                                            unsigned* state) {
+    if (blockIdx.x == 0 && threadIdx.x < kStateWords) state[threadIdx.x] = 0u;
+    const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
+    int v[kScanItems], s = 0;
+    load_items(ends, base, n, v);
+    for (int k = 0; k < kScanItems; ++k) s += v[k];
+    int run = tile_off[blockIdx.x] + block_scan(s) - s;
+    for (int k = 0; k < kScanItems; ++k) { run += v[k]; v[k] = run; }
+    if (base + kScanItems <= n && ((size_t)ends & 15) == 0) {
+        for (int k = 0; k < kScanItems; k += 4)
+            *reinterpret_cast<int4*>(ends + base + k) = make_int4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+    } else {
+        for (int k = 0; k < kScanItems; ++k)
+            if (base + k < n) ends[base + k] = v[k];
+    }
+}
+
+__global__ void scatter_kernel(const float* __restrict__ pos, int stride, int n, const int2* __restrict__ place,
+                               const int* __restrict__ ends, float4* __restrict__ sorted) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float* p = pos + (size_t)i * stride;
-        const int slot = atomicAdd(cursor + cell_of[i], 1);
-        sorted[slot] = make_float4(p[0], p[1], p[2], __int_as_float(i));
+        const int2 at = place[i];
+        sorted[__ldg(ends + at.x) - 1 - at.y] = make_float4(p[0], p[1], p[2], __int_as_float(i));
     }
 }
 
@@ -249,6 +293,20 @@ int grid_for(int n) {
     return std::max(1, std::min((n + kBlock - 1) / kBlock, std::max(sms, 1) * 8));
 }
 
+// The launches of one build (`state` all zero, as builds leave it).
+void launch_build(const float* positions, int stride, int n, float radius, float cell_factor, int table, float4* sorted,
+                  int* ends, float* params, int2* place, int* tile_sums, unsigned* state, cudaStream_t st) {
+    const int n_tiles = (table + kScanTile - 1) / kScanTile;
+    bounds_kernel<<<grid_for(std::max(n, table / 4)), kBlock, 0, st>>>(positions, stride, n, ends, table, radius,
+                                                                       cell_factor, params, state);
+    const int grid = grid_for(n);
+    if (n > 0) count_kernel<<<grid, kBlock, 0, st>>>(positions, stride, n, params, (uint32_t)table, ends, place);
+    scan_tiles_kernel<<<n_tiles, kBlock, 0, st>>>(ends, table, tile_sums, state);
+    scan_apply_kernel<<<n_tiles, kBlock, 0, st>>>(ends, table, tile_sums, state);
+    if (n > 0) scatter_kernel<<<grid, kBlock, 0, st>>>(positions, stride, n, place, ends, sorted);
+    note_launches(n > 0 ? 5 : 3);
+}
+
 // Grows geometrically: reallocation synchronizes the device, and a grid rebuilt every
 // iteration over a slowly growing photon count would otherwise reallocate every time.
 template <typename T>
@@ -288,9 +346,14 @@ imbart_hashgrid* imbart_hashgrid_create(int device) {
     int prev = 0;
     cudaGetDevice(&prev);
     cudaSetDevice(device);
-    const bool good = ok(cudaMalloc((void**)&g->params, sizeof(float) * 16), "cudaMalloc");
+    // The parameters, then the builds' state words, zero until the first build.
+    const bool good = ok(cudaMalloc((void**)&g->params, sizeof(float) * 16 + sizeof(unsigned) * kStateWords),
+                         "cudaMalloc") &&
+                      ok(cudaMemset(g->params, 0, sizeof(float) * 16 + sizeof(unsigned) * kStateWords), "cudaMemset") &&
+                      ok(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
     cudaSetDevice(prev);
-    if (!good) { delete g; return nullptr; }
+    if (!good) { cudaFree(g->params); delete g; return nullptr; }
+    g->state = reinterpret_cast<unsigned*>(g->params + 16);
     return g;
 }
 
@@ -299,8 +362,7 @@ void imbart_hashgrid_destroy(imbart_hashgrid* g) {
     int prev = 0;
     cudaGetDevice(&prev);
     cudaSetDevice(g->device);
-    cudaFree(g->sorted); cudaFree(g->cell_ends); cudaFree(g->cell_of); cudaFree(g->cursor);
-    cudaFree(g->block_sums); cudaFree(g->params);
+    cudaFree(g->sorted); cudaFree(g->cell_ends); cudaFree(g->place); cudaFree(g->block_sums); cudaFree(g->params);
     cudaSetDevice(prev);
     delete g;
 }
@@ -318,25 +380,12 @@ int imbart_hashgrid_build(imbart_hashgrid* g, const float* positions, int stride
     cudaSetDevice(g->device);
     int rc = 0;
     const int n_tiles = (table_size + kScanTile - 1) / kScanTile;
-    int* box = nullptr;
-    if (!grow(&g->sorted, &g->sorted_cap, n) || !grow(&g->cell_of, &g->cell_of_cap, n) ||
-        !grow(&g->cell_ends, &g->ends_cap, table_size) || !grow(&g->cursor, &g->cursor_cap, table_size) ||
-        !grow(&g->block_sums, &g->block_sums_cap, n_tiles + 8))
+    if (!grow(&g->sorted, &g->sorted_cap, n) || !grow(&g->place, &g->place_cap, n) ||
+        !grow(&g->cell_ends, &g->ends_cap, table_size) || !grow(&g->block_sums, &g->block_sums_cap, n_tiles))
         rc = IMBART_ERR_OUT_OF_MEMORY;
     if (!rc) {
-        box = g->block_sums + n_tiles;   // 6 ints after the tile sums
-        const int grid = grid_for(std::max(n, 1));
-        bbox_init_kernel<<<1, 32, 0, st>>>(box);
-        if (n > 0) bbox_kernel<<<grid, kBlock, 0, st>>>(positions, stride, n, box);
-        params_kernel<<<1, 32, 0, st>>>(box, radius, cell_factor, g->params);
-        ok(cudaMemsetAsync(g->cursor, 0, sizeof(int) * (size_t)table_size, st), "cudaMemsetAsync");
-        if (n > 0) count_kernel<<<grid, kBlock, 0, st>>>(positions, stride, n, g->params, (uint32_t)table_size,
-                                                         g->cursor, g->cell_of);
-        scan_tiles_kernel<<<n_tiles, kBlock, 0, st>>>(g->cursor, table_size, g->block_sums);
-        scan_sums_kernel<<<1, kBlock, 0, st>>>(g->block_sums, n_tiles);
-        scan_apply_kernel<<<n_tiles, kBlock, 0, st>>>(g->cursor, table_size, g->block_sums, g->cell_ends, g->cursor);
-        if (n > 0) scatter_kernel<<<grid, kBlock, 0, st>>>(positions, stride, n, g->cell_of, g->cursor, g->sorted);
-        note_launches(n > 0 ? 8 : 5);
+        launch_build(positions, stride, n, radius, cell_factor, table_size, g->sorted, g->cell_ends, g->params, g->place,
+                     g->block_sums, g->state, st);
         if (!ok(cudaGetLastError(), "hash grid build")) rc = IMBART_ERR_CUDA;
         g->n = n;
         g->table = table_size;
@@ -513,9 +562,9 @@ int imbart_hashgrid_get_arrays(const imbart_hashgrid* g, const void** sorted, co
 // fixed HBM budget accounts for every byte up front, and cudaMalloc / cudaFree synchronize
 // the device, stalling the other requests' streams; hosts that own all device memory
 // through their own arena hand out only buffers they sized themselves. For them the build's
-// scratch (bucket id per photon, bucket cursors, scan tile sums, bounding box) lives in one
+// scratch (bucket and place per photon, scan tile sums, state words) lives in one
 // statically sized device array below, held by every GPU that loads the library until the
-// process exits: 4 * (2^20 + 2^21 + 1024 + 8) bytes, about 12 MiB. The caller passes the
+// process exits: 4 * (2 * 2^20 + 1024 + 8) bytes, about 8 MiB. The caller passes the
 // inputs and the outputs it allocated itself.
 // ---------------------------------------------------------------------------------------
 namespace imbart {
@@ -523,7 +572,7 @@ namespace {
 constexpr int kNoAllocMaxPhotons = 1 << 20;
 constexpr int kNoAllocMaxTable = 1 << 21;
 constexpr int kNoAllocTiles = (kNoAllocMaxTable + kScanTile - 1) / kScanTile;
-constexpr size_t kNoAllocInts = (size_t)kNoAllocMaxPhotons + kNoAllocMaxTable + kNoAllocTiles + 8;
+constexpr size_t kNoAllocInts = 2 * (size_t)kNoAllocMaxPhotons + kNoAllocTiles + kStateWords;
 
 static __device__ __align__(256) int g_noalloc_scratch[kNoAllocInts];
 
@@ -566,26 +615,12 @@ extern "C" int imbart_hashgrid_build_noalloc(const float* positions, int stride,
         }
         scratch = g_noalloc_addr[device];
     }
-    int* cell_of = scratch;
-    int* cursor = cell_of + kNoAllocMaxPhotons;
-    int* tile_sums = cursor + kNoAllocMaxTable;
-    const int n_tiles = (table_size + kScanTile - 1) / kScanTile;
-    int* box = tile_sums + kNoAllocTiles;
-    float4* sorted = static_cast<float4*>(sorted_out);
-    cudaStream_t st = (cudaStream_t)stream;
-    const int grid = grid_for(std::max(n, 1));
-    // The scratch keeps the previous call's contents: the box and the bucket counts are
-    // reset here; bucket ids, tile sums and cursors are fully rewritten before they are read.
-    bbox_init_kernel<<<1, 32, 0, st>>>(box);
-    if (n > 0) bbox_kernel<<<grid, kBlock, 0, st>>>(positions, stride, n, box);
-    params_kernel<<<1, 32, 0, st>>>(box, radius, cell_factor, params_out);
-    if (!ok(cudaMemsetAsync(cursor, 0, sizeof(int) * (size_t)table_size, st), "cudaMemsetAsync")) return IMBART_ERR_CUDA;
-    if (n > 0) count_kernel<<<grid, kBlock, 0, st>>>(positions, stride, n, params_out, (uint32_t)table_size, cursor,
-                                                     cell_of);
-    scan_tiles_kernel<<<n_tiles, kBlock, 0, st>>>(cursor, table_size, tile_sums);
-    scan_sums_kernel<<<1, kBlock, 0, st>>>(tile_sums, n_tiles);
-    scan_apply_kernel<<<n_tiles, kBlock, 0, st>>>(cursor, table_size, tile_sums, cell_ends_out, cursor);
-    if (n > 0) scatter_kernel<<<grid, kBlock, 0, st>>>(positions, stride, n, cell_of, cursor, sorted);
-    note_launches(n > 0 ? 8 : 5);
+    int2* place = reinterpret_cast<int2*>(scratch);
+    int* tile_sums = scratch + 2 * kNoAllocMaxPhotons;
+    unsigned* state = reinterpret_cast<unsigned*>(tile_sums + kNoAllocTiles);
+    // The scratch keeps the previous call's contents: places and tile sums are fully rewritten
+    // before they are read, and a build leaves the state words zero as it found them.
+    launch_build(positions, stride, n, radius, cell_factor, table_size, static_cast<float4*>(sorted_out), cell_ends_out,
+                 params_out, place, tile_sums, state, (cudaStream_t)stream);
     return ok(cudaGetLastError(), "imbart_hashgrid_build_noalloc") ? 0 : IMBART_ERR_CUDA;
 }

@@ -338,7 +338,7 @@ int imbart_hashgrid_get_arrays(const imbart_hashgrid* grid, const void** sorted,
  * imbart_hashgrid_build, written to caller-owned DEVICE outputs: sorted_out (n float4: xyz +
  * photon index bits, in bucket order), cell_ends_out (table_size inclusive bucket ends) and
  * params_out (10 floats: lo xyz, hi xyz, radius, radius^2, cell size, 1/cell size). The build's
- * scratch is one static device array of about 12 MiB, held by every GPU that loads the library
+ * scratch is one static device array of about 8 MiB, held by every GPU that loads the library
  * until the process exits; it bounds n to 1,048,576 photons and table_size (<= 0: 2n) to
  * 2,097,152 buckets — larger requests return IMBART_ERR_LIMIT without launching anything.
  * The first call on a device looks the array's address up for that device
