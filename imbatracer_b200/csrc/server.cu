@@ -802,10 +802,8 @@ bool batched_wave(imbart_server* S) {
             for (Request* r : S->active_renders) kinds |= S->scenes[r->scene]->kind_mask;
             const bool group = __builtin_popcount(kinds) > 1;
             if (group) {
-                shade_key_multi_kernel<<<(n + 255) / 256, 256, 0, st>>>(S->d_reqs, S->d_scenes, S->req[cur], S->hits,
-                                                                         n, nullptr, S->keys);
-                launch_grouping(S->keys, n, nullptr, S->tile_counts, S->perm, st);
-                note_launches(1);
+                launch_grouping(MergedHitKeys{S->d_reqs, S->d_scenes, S->req[cur], S->hits}, n, nullptr, S->keys,
+                                S->tile_counts, S->perm, st);
                 p.perm = S->perm;
             }
             pt_shade_kernel<true><<<(n + 127) / 128, 128, 0, st>>>(p);

@@ -154,11 +154,14 @@ __global__ void light_gen_kernel(VcmParams p, const LightTile* tiles, int n_tile
 }
 
 // Material grouping keys of light-path slots (pt::shade_key; finished slots get key 7).
-__global__ void __launch_bounds__(256) light_key_kernel(ShadingScene s, const int4* __restrict__ hits,
-                                                        const float4* __restrict__ thrs, int n, uint8_t* keys) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) keys[i] = (uint8_t)(__float_as_int(thrs[i].w) < 0 ? 7 : pt::shade_key(s, hits[i]));
-}
+struct LightKeys {
+    ShadingScene s;
+    const int4* hits;
+    const float4* thrs;
+    __device__ __forceinline__ int operator()(int i) const {
+        return __float_as_int(thrs[i].w) < 0 ? 7 : pt::shade_key(s, hits[i]);
+    }
+};
 
 // connect_to_camera (vcm.cpp:260-320): a shadow ray towards the camera. Returns false when the
 // vertex does not project into the image or the BSDF cannot reach the camera.
@@ -878,10 +881,10 @@ bool ensure_shadow(imbart_vcm* v, long long need) {
     return good;
 }
 
-// The shading order of a wavefront of n paths: keys from `key_launch(keys)`, then the stable
-// counting sort into v->perm (pt::launch_grouping).
-template <typename KeyLaunch>
-bool group_paths(imbart_vcm* v, const imbart_shading* sh, int n, cudaStream_t s, KeyLaunch key_launch) {
+// The shading order of a wavefront of n paths: the stable counting sort of their keys into
+// v->perm (pt::launch_grouping).
+template <typename Keys>
+bool group_paths(imbart_vcm* v, const imbart_shading* sh, int n, cudaStream_t s, const Keys& key_of) {
     v->use_perm = __builtin_popcount(sh->kind_mask) > 1;    // one kind: nothing to group
     if (!v->use_perm) return true;
     if (v->sort_cap < n) {
@@ -891,9 +894,7 @@ bool group_paths(imbart_vcm* v, const imbart_shading* sh, int n, cudaStream_t s,
         v->sort_cap = good ? c : 0;
         if (!good) return false;
     }
-    key_launch(v->keys);
-    pt::launch_grouping(v->keys, n, nullptr, v->tile_counts, v->perm, s);
-    note_launches(1);
+    pt::launch_grouping(key_of, n, nullptr, v->keys, v->tile_counts, v->perm, s);
     return ok(cudaGetLastError(), "grouping kernels");
 }
 
@@ -1179,9 +1180,7 @@ int imbart_vcm_light_pass_range(imbart_vcm* v, const imbart_scene* scene, const 
         }
         p.cache = v->cache;
         if (!ok(cudaMemsetAsync(v->counts, 0, sizeof(int) * 4, s), "cudaMemsetAsync")) { rc = IMBART_ERR_CUDA; break; }
-        if (!group_paths(v, sh, n, s, [&](uint8_t* keys) {
-                light_key_kernel<<<(n + 255) / 256, 256, 0, s>>>(p.s, v->l_hits, v->l_thr, n, keys);
-            })) {
+        if (!group_paths(v, sh, n, s, LightKeys{p.s, v->l_hits, v->l_thr})) {
             rc = IMBART_ERR_CUDA;
             break;
         }
@@ -1326,9 +1325,7 @@ int imbart_vcm_camera_pass_range(imbart_vcm* v, const imbart_scene* scene, const
             ++n_waves;
             if (!ok(cudaMemsetAsync(v->counts, 0, sizeof(int) * 4, s), "cudaMemsetAsync")) { rc = IMBART_ERR_CUDA; break; }
             const int nxt = 1 - cur;
-            if (!group_paths(v, sh, n, s, [&](uint8_t* keys) {
-                    pt::shade_key_kernel<<<(n + 255) / 256, 256, 0, s>>>(p.s, v->c_hits, n, nullptr, keys);
-                })) {
+            if (!group_paths(v, sh, n, s, pt::HitKeys{p.s, v->c_hits})) {
                 rc = IMBART_ERR_CUDA;
                 break;
             }

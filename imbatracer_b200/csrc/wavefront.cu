@@ -334,10 +334,9 @@ int build_range_graph(imbart_pt_context* ctx, const imbart_scene* scene, const i
         p.counts = out;
         p.image = image;
         if (group) {
-            main = gb.kernel({main}, shade_key_kernel, dim3(small_grid), dim3(256), sh->s, ctx->hits, n, n_in,
-                             ctx->keys);
             const int tiles = group_tiles(n);
-            main = gb.kernel({main}, group_count_kernel, dim3(tiles), dim3(256), ctx->keys, n, n_in, ctx->tile_counts);
+            main = gb.kernel({main}, group_count_kernel<HitKeys>, dim3(tiles), dim3(256), HitKeys{sh->s, ctx->hits}, n,
+                             n_in, ctx->keys, ctx->tile_counts);
             main = gb.kernel({main}, group_scan_kernel, dim3(1), dim3(1024), ctx->tile_counts, n, n_in);
             main = gb.kernel({main}, group_scatter_kernel, dim3(tiles), dim3(256), ctx->keys, n, n_in,
                              ctx->tile_counts, ctx->perm);
@@ -687,9 +686,7 @@ int imbart_pt_render_range(imbart_pt_context* ctx, const imbart_scene* scene, co
             p.image = image;
             if (group) {
                 // Group the wavefront's paths by material kind before shading.
-                shade_key_kernel<<<(n + 255) / 256, 256, 0, st>>>(sh->s, ctx->hits, n, nullptr, ctx->keys);
-                launch_grouping(ctx->keys, n, nullptr, ctx->tile_counts, ctx->perm, st);
-                note_launches(1);
+                launch_grouping(HitKeys{sh->s, ctx->hits}, n, nullptr, ctx->keys, ctx->tile_counts, ctx->perm, st);
                 p.perm = ctx->perm;
             }
             pt_shade_kernel<false><<<(n + 127) / 128, 128, 0, st>>>(p);
@@ -750,10 +747,12 @@ int imbart_group_by_key(const unsigned char* keys, int n, int* perm, void* strea
     }
     if (n == 0) return 0;
     cudaStream_t st = (cudaStream_t)stream;
+    // Scratch: 8 ints per tile, then a byte per entry.
     int* tiles = nullptr;
-    if (!ok(cudaMallocAsync((void**)&tiles, sizeof(int) * kShadeKeys * group_tiles(n), st), "cudaMallocAsync"))
+    const size_t counts = (size_t)kShadeKeys * group_tiles(n);
+    if (!ok(cudaMallocAsync((void**)&tiles, sizeof(int) * counts + (size_t)n, st), "cudaMallocAsync"))
         return IMBART_ERR_OUT_OF_MEMORY;
-    launch_grouping(keys, n, nullptr, tiles, perm, st);
+    launch_grouping(GivenKeys{keys}, n, nullptr, reinterpret_cast<uint8_t*>(tiles + counts), tiles, perm, st);
     const bool good = ok(cudaGetLastError(), "grouping kernels");
     cudaFreeAsync(tiles, st);
     return good ? 0 : IMBART_ERR_CUDA;
