@@ -145,16 +145,21 @@ imbart_scene* prepare(Convert convert, int root, const Node* nodes, int n_nodes,
 // ---------------------------------------------------------------------------------------
 // Three query classes keep their own variant and refill threshold: incoherent closest hit,
 // any hit, and closest hit over coherent rays (camera rays, flag IMBART_TRACE_COHERENT),
-// which traverse best in static batches (refill only when the whole warp is idle).
+// which traverse best in nearly static batches (refill when most of the warp is idle).
 constexpr int kTraceVariants = 17;   // persistent-kernel shapes 1..17 (0: one ray per thread)
 constexpr int kFirstCoopVariant = 11; // 11..17: the shapes with the cooperative triangle phase
 
 // Each class also keeps its triangle batch: in the per-lane shapes, the triangles a lane
 // tests per loop trip before the lanes with node work take their next node step (0: the
 // whole group at once; two measured best there: secondary rays +13 %, camera rays +7 % over
-// 0); the cooperative shapes ignore it. Defaults: the cooperative 256 x 3 shape for every
-// class (on the frame's ray sets of the instanced scene: camera / secondary / shadow rays
-// +2 / +9 / +10 % over the best per-lane shapes).
+// 0); the cooperative shapes ignore it. Defaults: cooperative shapes for every class (on the
+// frame's ray sets of the instanced scene: camera / secondary / shadow rays +2 / +9 / +10 % over
+// the best per-lane shapes). Incoherent closest hits: 128 x 7, refill at 8 idle lanes (1 M random
+// rays over 201 instances 0.90 ms at 8, 0.89 at 4 and 6, 0.93 at 12, 1.24 at 24; over one mesh
+// 0.181 at 8 and 12, 0.187 at 4; the 256 x 3 shape is 1 % behind on each). Any hit: 256 x 3 at 8
+// (a 1080p frame of the instanced scene 18.26 ms; 18.30 with 128 x 7, which is 4 % ahead on
+// 2 M shadow rays over one masked mesh). Camera rays: 256 x 3 at 24 (the frame 18.20 ms; 18.26
+// at 32, 18.56 at 16).
 struct TraceConfig {
     int variant, refill, postpone, variant_any;
     int refill_any, variant_coh, refill_coh;
@@ -163,7 +168,7 @@ struct TraceConfig {
 
 std::mutex g_cfg_mutex;
 bool g_cfg_init = false;
-TraceConfig g_cfg{11, 24, 0, 11, 8, 11, 32};
+TraceConfig g_cfg{17, 8, 0, 11, 8, 11, 24};
 
 int env_int(const char* name, int dflt) {
     const char* v = getenv(name);

@@ -68,6 +68,24 @@ struct TraceParams {
     int direct_inst;
 };
 
+// The cooperative kernels issue at 70-75 % of the SMs' rate, but on incoherent rays only 13.6 of a
+// warp's 32 lanes take part in an instruction (ncu, 1 M rays over 201 instances), so they choose
+// when a warp does what:
+//  * an instance entry waits while fewer than kWaitEnter lanes stand at one, and the triangle phase
+//    while its groups hold fewer than kWaitPairs pairs, as long as kWaitReady lanes can take
+//    another node step meanwhile. Each ray still does the same steps in the same order.
+//  * a warp refills once a few lanes are idle (the classes' defaults in trace.cu).
+// Refills at 4-8 idle lanes instead of 24 took those rays from 1.25 to 1.00 ms, the waits to
+// 0.90 ms (17.7 lanes); entries at 4 or 12 lanes, pairs at 24 or 32 and 12 ready lanes measured
+// 1-8 % slower. Camera rays and shadow rays gain 3 %.
+constexpr int kWaitEnter = 8, kWaitPairs = 16, kWaitReady = 8;
+// A queue that gives a resident warp at most kShortShare rays is spread over all of them, each
+// with its share of lanes; the triangle phase still has the whole warp. The chain of the
+// longest ray bounds such a launch, and a warp with fewer rays passes through its trips sooner:
+// 2,049 rays 47 -> 35 us, 8,000 57 -> 47 us, 20,000 58 -> 55 us. Above that the warps are better
+// filled (50,000 rays, share 15: 72 -> 73 us; 201 instances 194 -> 199 us).
+constexpr int kShortShare = 8;
+
 constexpr uint32_t kEntryTri = 3u;      // triangle group (postponed): x = prim base, y = prim mask
 
 // Work counters of one ray, accumulated only by the statistics variant of the kernel.
@@ -474,6 +492,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) trace_persistent(TracePara
     constexpr int kCW = kCoop ? kBlock / 32 : 1;     // warps with cooperative-phase slots
     __shared__ uint2 sstack[kSh][kBlock];
     __shared__ uint32_t s_key[kCW][32];              // per owner lane: smallest key of a pass
+    __shared__ int s_own[kCW][32];                   // owner lanes in order
     __shared__ int s_tri[kCW][32];                   // per owner lane: its winning triangle id
     __shared__ float4 s_hit[kCW][32];                // per owner lane: the winner's t, u, v
     // The world ray (origin, direction, inverse direction, pad, octant): instance entries read
@@ -502,6 +521,9 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) trace_persistent(TracePara
     r.Sx = r.Sy = r.Sz = 0.0f;
     r.kx = r.ky = r.kz = 0;
     const int count = p.count_ptr ? min(__ldg(p.count_ptr), p.count) : p.count;
+    // Short queues (kShortShare): lanes beyond the warp's share of the rays stay out.
+    const int share = (int)(((long long)count + p.total_warps - 1) / p.total_warps);
+    if (kCoop && share <= kShortShare && (int)lane >= share) ray = count;
 
     auto push = [&](uint32_t x, uint32_t y) -> bool {
         if (sp >= kStackSize) return false;
@@ -596,6 +618,14 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) trace_persistent(TracePara
             }
         }
 
+        // With few lanes at an instance and others that can go on without it, the entry waits
+        // (kWaitReady).
+        bool wait_enter = false;
+        if (kCoop && !kFlat) {
+            const unsigned enter = __ballot_sync(kFull, !next && t_mask != 0 && !bottom);
+            const unsigned ready = __ballot_sync(kFull, !next && t_mask == 0);
+            wait_enter = __popc(enter) < kWaitEnter && __popc(ready) >= kWaitReady;
+        }
         // Primitive step: instance entry, and per-lane triangle tests.
         if (!next && t_mask != 0) {
             if (kFlat || bottom) {
@@ -638,7 +668,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) trace_persistent(TracePara
                     }
                     if (stop) { finish(); next = true; }
                 }
-            } else {
+            } else if (!wait_enter) {
                 // Enter the next instance of the group.
                 const uint32_t i = __ffs(t_mask) - 1;
                 t_mask &= t_mask - 1;
@@ -675,106 +705,113 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) trace_persistent(TracePara
         // Cooperative triangle phase (every lane of the warp takes part).
         if (kCoop) {
             const bool want = !next && (kFlat || bottom) && t_mask != 0;
-            if (__ballot_sync(kFull, want) != 0u) {
+            const int cnt = want ? __popc(t_mask) : 0;
+            const unsigned wm = __ballot_sync(kFull, want);
+            const unsigned ready = __ballot_sync(kFull, !next && t_mask == 0);
+            if (wm != 0u) {
                 const int w = tid >> 5;
-                const int cnt = want ? __popc(t_mask) : 0;
-                int incl = cnt;
+                // Pairs before this lane's, from ballots of the counts' bits (at most 24 each).
+                int excl = 0, total = 0;
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int y = __shfl_up_sync(kFull, incl, o);
-                    if ((int)lane >= o) incl += y;
+                for (int bit = 0; bit < 5; ++bit) {
+                    const unsigned m = __ballot_sync(kFull, (cnt >> bit) & 1);
+                    excl += __popc(m & lt_mask) << bit;
+                    total += __popc(m) << bit;
                 }
-                const int total = __shfl_sync(kFull, incl, 31);
-                const int excl = incl - cnt;
-                const uint32_t kpack = (uint32_t)r.kx | ((uint32_t)r.ky << 2) | ((uint32_t)r.kz << 4);
-                int found_k = -1;    // any hit: position of the group's first accepted triangle
-                for (int pass = 0; pass < total; pass += 32) {
-                    const int j = pass + (int)lane;
-                    // Owner of pair j: the first lane whose inclusive count exceeds j.
-                    int o = 0;
-#pragma unroll
-                    for (int step = 16; step >= 1; step >>= 1) {
-                        const int c = __shfl_sync(kFull, incl, o + step - 1);
-                        if (c <= j) o += step;
-                    }
-                    const int o_excl = __shfl_sync(kFull, excl, o);
-                    const uint32_t o_mask = __shfl_sync(kFull, t_mask, o);
-                    const uint32_t o_base = __shfl_sync(kFull, t_base, o);
-                    SpaceRay q;
-                    q.ox = __shfl_sync(kFull, r.ox, o);
-                    q.oy = __shfl_sync(kFull, r.oy, o);
-                    q.oz = __shfl_sync(kFull, r.oz, o);
-                    q.Sx = __shfl_sync(kFull, r.Sx, o);
-                    q.Sy = __shfl_sync(kFull, r.Sy, o);
-                    q.Sz = __shfl_sync(kFull, r.Sz, o);
-                    const uint32_t qk = __shfl_sync(kFull, kpack, o);
-                    q.kx = (int)(qk & 3u); q.ky = (int)((qk >> 2) & 3u); q.kz = (int)((qk >> 4) & 3u);
-                    const float o_tmin = __shfl_sync(kFull, tmin, o);
-                    const float o_best = __shfl_sync(kFull, best_t, o);
-                    const bool has = j < total;
-                    const int k = j - o_excl;
-                    const int ti = has ? (int)(o_base + nth_set_bit(o_mask, k)) : -1;
-                    float4 a, b, c;
-                    if (has) {
-                        const float4* tp = reinterpret_cast<const float4*>(p.tris + ti);
-                        a = __ldg(tp + 0); b = __ldg(tp + 1); c = __ldg(tp + 2);
-                    }
-                    bool cand = false;
-                    float t = 0.0f, u = 0.0f, v = 0.0f;
-                    int tri = 0;
-                    if (has && tri_test(q, a, b, c, t, u, v) && t >= o_tmin && t <= o_best) {
-                        tri = __float_as_int(a.w);
-                        cand = !kMasked || mask_opaque(p, tri, u, v);
-                    }
-                    const bool in_pass = want && excl < pass + 32 && incl > pass;
-                    if (in_pass) { s_key[w][lane] = 0xffffffffu; s_tri[w][lane] = 0x7fffffff; }
+                if (!(total < kWaitPairs && __popc(ready) >= kWaitReady)) {
+                    const int incl = excl + cnt;
+                    if (want) s_own[w][__popc(wm & lt_mask)] = (int)lane;
                     __syncwarp();
-                    uint32_t key;
-                    if (kAnyHit) {
-                        key = (uint32_t)k;            // the group's test order
-                    } else {
-                        // t as an ordered unsigned key (+0 and -0 equal, as the tie rule has it)
-                        const uint32_t tb = __float_as_uint(__fadd_rn(t, 0.0f));
-                        key = (tb & 0x80000000u) ? ~tb : (tb | 0x80000000u);
-                    }
-                    if (cand) atomicMin(&s_key[w][o], key);
-                    __syncwarp();
-                    bool win = cand && s_key[w][o] == key;
-                    if (!kAnyHit) {
-                        if (win) atomicMin(&s_tri[w][o], tri);
+                    int started = -1;    // owners before the pass, less one
+                    const uint32_t kpack = (uint32_t)r.kx | ((uint32_t)r.ky << 2) | ((uint32_t)r.kz << 4);
+                    int found_k = -1;    // any hit: position of the group's first accepted triangle
+                    for (int pass = 0; pass < total; pass += 32) {
+                        const int j = pass + (int)lane;
+                        // Owner of pair j: the last one whose pairs start at or before it.
+                        const unsigned start = want && (unsigned)(excl - pass) < 32u ? 1u << (excl - pass) : 0u;
+                        const unsigned starts = __reduce_or_sync(kFull, start);
+                        const int o = s_own[w][started + __popc(starts & (lt_mask | (1u << lane)))];
+                        started += __popc(starts);
+                        const int o_excl = __shfl_sync(kFull, excl, o);
+                        const uint32_t o_mask = __shfl_sync(kFull, t_mask, o);
+                        const uint32_t o_base = __shfl_sync(kFull, t_base, o);
+                        SpaceRay q;
+                        q.ox = __shfl_sync(kFull, r.ox, o);
+                        q.oy = __shfl_sync(kFull, r.oy, o);
+                        q.oz = __shfl_sync(kFull, r.oz, o);
+                        q.Sx = __shfl_sync(kFull, r.Sx, o);
+                        q.Sy = __shfl_sync(kFull, r.Sy, o);
+                        q.Sz = __shfl_sync(kFull, r.Sz, o);
+                        const uint32_t qk = __shfl_sync(kFull, kpack, o);
+                        q.kx = (int)(qk & 3u); q.ky = (int)((qk >> 2) & 3u); q.kz = (int)((qk >> 4) & 3u);
+                        const float o_tmin = __shfl_sync(kFull, tmin, o);
+                        const float o_best = __shfl_sync(kFull, best_t, o);
+                        const bool has = j < total;
+                        const int k = j - o_excl;
+                        const int ti = has ? (int)(o_base + nth_set_bit(o_mask, k)) : -1;
+                        float4 a, b, c;
+                        if (has) {
+                            const float4* tp = reinterpret_cast<const float4*>(p.tris + ti);
+                            a = __ldg(tp + 0); b = __ldg(tp + 1); c = __ldg(tp + 2);
+                        }
+                        bool cand = false;
+                        float t = 0.0f, u = 0.0f, v = 0.0f;
+                        int tri = 0;
+                        if (has && tri_test(q, a, b, c, t, u, v) && t >= o_tmin && t <= o_best) {
+                            tri = __float_as_int(a.w);
+                            cand = !kMasked || mask_opaque(p, tri, u, v);
+                        }
+                        if (__ballot_sync(kFull, cand) == 0u) continue;
+                        const bool in_pass = want && excl < pass + 32 && incl > pass;
+                        if (in_pass) { s_key[w][lane] = 0xffffffffu; s_tri[w][lane] = 0x7fffffff; }
                         __syncwarp();
-                        win = win && s_tri[w][o] == tri;
-                    }
-                    if (win) {
-                        if (kAnyHit) s_tri[w][o] = tri;
-                        s_hit[w][o] = make_float4(t, u, v, 0.0f);
-                    }
-                    __syncwarp();
-                    if (in_pass && s_key[w][lane] != 0xffffffffu) {
-                        const int tc = s_tri[w][lane];
-                        const float4 hv = s_hit[w][lane];
+                        uint32_t key;
                         if (kAnyHit) {
-                            if (found_k < 0) {
-                                found_k = (int)s_key[w][lane];
-                                best_t = hv.x; s_uv[0][tid] = hv.y; s_uv[1][tid] = hv.z; best_tri = tc; best_inst = cur_inst;
-                            }
+                            key = (uint32_t)k;            // the group's test order
                         } else {
-                            const bool closer = (hv.x < best_t) ||
-                                (hv.x == best_t && (kFlat ? (best_tri < 0 || tc < best_tri)
-                                                          : (best_tri < 0 || cur_inst < best_inst ||
-                                                             (cur_inst == best_inst && tc < best_tri))));
-                            if (closer) {
-                                best_t = hv.x; s_uv[0][tid] = hv.y; s_uv[1][tid] = hv.z; best_tri = tc; best_inst = cur_inst;
-                                tlimit = best_t * IMBART_SLACK;
+                            // t as an ordered unsigned key (+0 and -0 equal, as the tie rule has it)
+                            const uint32_t tb = __float_as_uint(__fadd_rn(t, 0.0f));
+                            key = (tb & 0x80000000u) ? ~tb : (tb | 0x80000000u);
+                        }
+                        if (cand) atomicMin(&s_key[w][o], key);
+                        __syncwarp();
+                        bool win = cand && s_key[w][o] == key;
+                        if (!kAnyHit) {
+                            if (win) atomicMin(&s_tri[w][o], tri);
+                            __syncwarp();
+                            win = win && s_tri[w][o] == tri;
+                        }
+                        if (win) {
+                            if (kAnyHit) s_tri[w][o] = tri;
+                            s_hit[w][o] = make_float4(t, u, v, 0.0f);
+                        }
+                        __syncwarp();
+                        if (in_pass && s_key[w][lane] != 0xffffffffu) {
+                            const int tc = s_tri[w][lane];
+                            const float4 hv = s_hit[w][lane];
+                            if (kAnyHit) {
+                                if (found_k < 0) {
+                                    found_k = (int)s_key[w][lane];
+                                    best_t = hv.x; s_uv[0][tid] = hv.y; s_uv[1][tid] = hv.z; best_tri = tc; best_inst = cur_inst;
+                                }
+                            } else {
+                                const bool closer = (hv.x < best_t) ||
+                                    (hv.x == best_t && (kFlat ? (best_tri < 0 || tc < best_tri)
+                                                              : (best_tri < 0 || cur_inst < best_inst ||
+                                                                 (cur_inst == best_inst && tc < best_tri))));
+                                if (closer) {
+                                    best_t = hv.x; s_uv[0][tid] = hv.y; s_uv[1][tid] = hv.z; best_tri = tc; best_inst = cur_inst;
+                                    tlimit = best_t * IMBART_SLACK;
+                                }
                             }
                         }
+                        __syncwarp();
                     }
-                    __syncwarp();
-                }
-                if (want) {
-                    if (kStats) st.tris += (kAnyHit && found_k >= 0) ? (uint32_t)(found_k + 1) : (uint32_t)cnt;
-                    t_mask = 0;
-                    if (kAnyHit && found_k >= 0) { finish(); next = true; }
+                    if (want) {
+                        if (kStats) st.tris += (kAnyHit && found_k >= 0) ? (uint32_t)(found_k + 1) : (uint32_t)cnt;
+                        t_mask = 0;
+                        if (kAnyHit && found_k >= 0) { finish(); next = true; }
+                    }
                 }
             }
         }
