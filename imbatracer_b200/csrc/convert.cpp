@@ -8,9 +8,9 @@
 // is the top-level root (scene.cpp:167-188), instance nodes point at mesh roots (`next`).
 //
 // The conversion parses the reachable tree into an intermediate binary/n-ary tree, splits
-// leaves into runs of at most three primitives, collapses the tree into 8-wide nodes
-// (repeatedly opening the child with the largest surface area), assigns child slots by
-// direction octant and quantizes child boxes conservatively to 8 bits per plane.
+// leaves into runs of at most three primitives, collapses the tree into 8-wide nodes (of mesh
+// trees those of smallest summed surface area, Collapse below), assigns child slots by direction
+// octant and quantizes child boxes conservatively to 8 bits per plane.
 // The node width is 8 or 4 (imbart_set_node_width): a 4-wide tree uses slots 0..3 of the
 // same 80-byte record, ordered by the x/y quadrant, and leaves slots 4..7 empty.
 #include <algorithm>
@@ -81,10 +81,11 @@ struct IBox {
     }
 };
 
-// Intermediate tree node: internal (children) or leaf (a run of primitives).
+// Intermediate binary tree node: internal (two children, which precede it in the tree's array)
+// or leaf (a run of primitives).
 struct INode {
     IBox box;
-    std::vector<int> kids;
+    int kids[2] = {-1, -1};
     int pbegin = 0, pcount = 0;  // leaf: indices into the tree's prim list
     bool leaf() const { return pcount > 0; }
 };
@@ -144,7 +145,8 @@ int add_leaf(ITree& tree, int first, int n, const IBox& leaf_box, PrimBox prim_b
     const int r = add_leaf(tree, first + half, n - half, rb, prim_box);
     INode nd;
     nd.box = leaf_box;
-    nd.kids = {l, r};
+    nd.kids[0] = l;
+    nd.kids[1] = r;
     tree.nodes.push_back(nd);
     return (int)tree.nodes.size() - 1;
 }
@@ -153,32 +155,97 @@ int add_leaf(ITree& tree, int first, int n, const IBox& leaf_box, PrimBox prim_b
 // Collapse into 8-wide nodes
 // ---------------------------------------------------------------------------------------
 
-struct WideBuilder {
-    std::vector<WideNode>& out;
-    int width;   // children per node: 8, or 4 (slots 0..3)
-    WideBuilder(std::vector<WideNode>& o, int w) : out(o), width(w == 4 ? 4 : 8) {}
+// Which binary nodes become wide nodes: the choice with the smallest sum of wide-node surface
+// areas (the expected node visits of a random ray), by dynamic programming as in Ylitie, Karras
+// and Laine, "Efficient Incoherent Ray Traversal on GPUs Through Compressed Wide BVHs" (HPG
+// 2017), section 3.1. cost[m - 1] of a node is the smallest sum below it when it may take up to
+// m entries of the wide node above: as one entry (a leaf, or a wide node of its own) or, for
+// split[m - 1] = k > 0, through its children with k and m - k. Opening the child of largest area
+// first left 4.2-4.3 of 8 slots filled; this fills 5.8-6.2, with a third fewer nodes.
+// Measured (B200): 1 M random rays over 201 instances 936 -> 913 us, the 1080p frame (4 samples)
+// 18.57 -> 18.25 ms, a VCM iteration over 2 M triangles 13.9 -> 13.5 ms, 512 k triangles refitted
+// and 65,536 rays traced 270 -> 231 us.
+// The top level keeps opening the largest child: a ray enters the instances of a node in slot
+// order, not by distance, and fuller nodes made camera rays enter 4.53 instead of 4.32 of them
+// (the frame was 1 % slower).
+struct Collapse {
+    struct Choice {
+        float cost[8];
+        uint8_t split[8];
+    };
+    std::vector<Choice> at;
+    int width;
 
-    // Children of a wide node: open the internal child with the largest area until `width`.
-    static std::vector<int> gather(const ITree& t, int n, int width) {
-        std::vector<int> kids;
-        if (t.nodes[n].leaf()) { kids.push_back(n); return kids; }
-        kids = t.nodes[n].kids;
-        while ((int)kids.size() < width) {
-            int best = -1; float best_area = -1.0f;
-            for (int i = 0; i < (int)kids.size(); ++i) {
-                const INode& k = t.nodes[kids[i]];
+    Collapse(const ITree& t, int w, bool largest_first) : at(largest_first ? 0 : t.nodes.size()), width(w) {
+        if (largest_first) return;
+        for (size_t n = 0; n < t.nodes.size(); ++n) {
+            const INode& nd = t.nodes[n];
+            Choice& c = at[n];
+            if (nd.leaf()) {
+                for (int m = 0; m < 8; ++m) { c.cost[m] = 0.0f; c.split[m] = 0; }
+                continue;
+            }
+            const Choice &l = at[nd.kids[0]], &r = at[nd.kids[1]];
+            for (int m = 2; m <= width; ++m) {
+                float best = l.cost[0] + r.cost[m - 2];
+                int k = 1;
+                for (int j = 2; j < m; ++j) {
+                    const float v = l.cost[j - 1] + r.cost[m - j - 1];
+                    if (v < best) { best = v; k = j; }
+                }
+                c.cost[m - 1] = best;
+                c.split[m - 1] = (uint8_t)k;
+            }
+            c.cost[0] = nd.box.half_area() + c.cost[width - 1];
+            c.split[0] = 0;
+            // The entry counts below the full width may prefer a wide node of its own; the full
+            // width's split stays, it is how that wide node takes its children.
+            for (int m = 2; m < width; ++m)
+                if (c.cost[0] <= c.cost[m - 1]) { c.cost[m - 1] = c.cost[0]; c.split[m - 1] = 0; }
+        }
+    }
+
+    // Children of wide node n.
+    void children(const ITree& t, int n, std::vector<int>& out) const {
+        out.clear();
+        if (t.nodes[n].leaf()) out.push_back(n);
+        else if (at.empty()) open_largest(t, n, out);
+        else open(t, n, width, out);
+    }
+
+    void open_largest(const ITree& t, int n, std::vector<int>& out) const {
+        out.assign(t.nodes[n].kids, t.nodes[n].kids + 2);
+        while ((int)out.size() < width) {
+            int best = -1;
+            float best_area = -1.0f;
+            for (int i = 0; i < (int)out.size(); ++i) {
+                const INode& k = t.nodes[out[i]];
                 if (k.leaf()) continue;
-                if ((int)(kids.size() - 1 + k.kids.size()) > width) continue;
                 const float a = k.box.half_area();
                 if (a > best_area) { best_area = a; best = i; }
             }
             if (best < 0) break;
-            const std::vector<int> sub = t.nodes[kids[best]].kids;
-            kids.erase(kids.begin() + best);
-            kids.insert(kids.end(), sub.begin(), sub.end());
+            const INode& k = t.nodes[out[best]];
+            out.erase(out.begin() + best);
+            out.insert(out.end(), k.kids, k.kids + 2);
         }
-        return kids;
     }
+
+    void open(const ITree& t, int n, int m, std::vector<int>& out) const {
+        const int k = at[n].split[m - 1];
+        const int share[2] = {k, m - k};
+        for (int j = 0; j < 2; ++j) {
+            const int x = t.nodes[n].kids[j];
+            if (t.nodes[x].leaf() || at[x].split[share[j] - 1] == 0) out.push_back(x);
+            else open(t, x, share[j], out);
+        }
+    }
+};
+
+struct WideBuilder {
+    std::vector<WideNode>& out;
+    int width;   // children per node: 8, or 4 (slots 0..3)
+    WideBuilder(std::vector<WideNode>& o, int w) : out(o), width(w == 4 ? 4 : 8) {}
 
     // Greedy slot assignment: slot s prefers children towards (s&1?+x:-x, s&2?+y:-y, s&4?+z:-z);
     // a 4-wide node uses slots 0..3, ordered by x and y alone.
@@ -261,15 +328,17 @@ struct WideBuilder {
     // Builds the wide tree of `t` rooted at intermediate node `root`. Leaf primitives are
     // appended through `emit(prim)` which returns the index of the emitted record.
     template <typename Emit>
-    int build(const ITree& t, int root, Emit emit) {
+    int build(const ITree& t, int root, bool top_level, Emit emit) {
         const int wroot = (int)out.size();
         out.emplace_back();
+        const Collapse collapse(t, width, top_level);
+        std::vector<int> kids;
         std::deque<std::pair<int, int>> work;
         work.push_back({wroot, root});
         while (!work.empty()) {
             auto [w, n] = work.front();
             work.pop_front();
-            std::vector<int> kids = gather(t, n, width);
+            collapse.children(t, n, kids);
             int slot_of[8];
             assign_slots(t, kids, width, slot_of);
             int kid_in_slot[8];
@@ -417,9 +486,26 @@ struct Parser {
         }
         if (parsed.empty()) { err = "BVH node without children"; return -1; }
         if (parsed.size() == 1) return parsed[0];   // single-leaf wrapper
+        // More than two children (the four-wide layout) become a small binary tree: neighbours
+        // pair up, the last pair is the node itself.
+        while (parsed.size() > 2) {
+            std::vector<int> pairs;
+            for (size_t i = 0; i < parsed.size(); i += 2) {
+                if (i + 1 == parsed.size()) { pairs.push_back(parsed[i]); break; }
+                INode nd;
+                nd.box = tree.nodes[parsed[i]].box;
+                nd.box.grow(tree.nodes[parsed[i + 1]].box);
+                nd.kids[0] = parsed[i];
+                nd.kids[1] = parsed[i + 1];
+                tree.nodes.push_back(nd);
+                pairs.push_back((int)tree.nodes.size() - 1);
+            }
+            parsed = pairs;
+        }
         INode nd;
         nd.box = box;
-        nd.kids = parsed;
+        nd.kids[0] = parsed[0];
+        nd.kids[1] = parsed[1];
         tree.nodes.push_back(nd);
         return (int)tree.nodes.size() - 1;
     }
@@ -483,7 +569,7 @@ std::string convert_common(int root, int n_nodes, const imbart_instance_node* in
             out.tris.push_back(parsed[rec - tris_before]);
             return (int)out.tris.size() - 1;
         };
-        wide_root_of[mroot] = wb.build(bt, br, emit_tri);
+        wide_root_of[mroot] = wb.build(bt, br, false, emit_tri);
     }
 
     // Top level.
@@ -498,7 +584,7 @@ std::string convert_common(int root, int n_nodes, const imbart_instance_node* in
         out.insts.push_back(wi);
         return (int)out.insts.size() - 1;
     };
-    out.root = wb.build(top, top_root, emit_inst);
+    out.root = wb.build(top, top_root, true, emit_inst);
     out.top_nodes = (int)out.nodes.size() - top_first;
     if (out.nodes.size() >= (size_t)1 << 30 || out.tris.size() >= (size_t)1 << 30 ||
         out.insts.size() >= (size_t)1 << 30)

@@ -17,11 +17,12 @@
 //      does not depend on thread timing. A merge also computes the node's surface-area cost
 //      (traversal cost 1, one unit per primitive) and turns subtrees of at most three triangles
 //      into leaves where that is cheaper (one instance per leaf at the top level);
+//      It also chooses the collapse below it: the wide nodes of smallest summed surface area, by
+//      the dynamic programme of the host converter (convert.cpp, Collapse);
 //   4. a top-down collapse into 8-wide nodes, level by level over all meshes, then over the
-//      instances: a wide node takes its binary node's children and opens the largest-area
-//      internal child until it has 8, assigns slots by direction octant, quantizes the child
-//      boxes conservatively (the same arithmetic as the host converter, convert.cpp) and writes
-//      the leaves' triangle or instance records.
+//      instances: a wide node takes the chosen descendants of its binary node as children,
+//      assigns slots by direction octant, quantizes the child boxes conservatively (the same
+//      arithmetic as the host converter) and writes the leaves' triangle or instance records.
 // Hits do not depend on the tree: traversal over this layout finds the same closest hit
 // as over any other BVH of the same triangles.
 //
@@ -318,11 +319,50 @@ struct Forest {
     int* cnt;               //   primitives
     float* cost;            //   surface-area cost
     uint8_t* leafy;         //   becomes a leaf
+    float* area;            //   7 each: smallest sum of wide-node areas below with up to m entries
+    uint8_t* split;         //   8 each: entries of the left child with m entries (0: one entry)
     int* roots;             // per segment
 };
 
 __device__ __forceinline__ bool is_leafy(const Forest& f, int node) { return node < f.n || f.leafy[node - f.n] != 0; }
 __device__ __forceinline__ int prim_count(const Forest& f, int node) { return node < f.n ? 1 : f.cnt[node - f.n]; }
+
+// The collapse below new inner node k (children l, r, half area a): area[7 k + m - 1] and
+// split[8 k + m - 1] for m entries, as convert.cpp's Collapse.
+__device__ __forceinline__ void choose_collapse(const Forest& f, int k, int l, int r, bool leaf, float a) {
+    float* out = f.area + 7ll * k;
+    uint8_t split[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    float cost[8];
+    for (int m = 0; m < 8; ++m) cost[m] = 0.0f;
+    if (!leaf) {
+        float lc[7], rc[7];
+        const bool li = !is_leafy(f, l), ri = !is_leafy(f, r);
+        for (int m = 0; m < 7; ++m) {
+            lc[m] = li ? f.area[7ll * (l - f.n) + m] : 0.0f;
+            rc[m] = ri ? f.area[7ll * (r - f.n) + m] : 0.0f;
+        }
+#pragma unroll
+        for (int m = 2; m <= 8; ++m) {
+            float best = lc[0] + rc[m - 2];
+            int s = 1;
+#pragma unroll
+            for (int j = 2; j < m; ++j) {
+                const float v = lc[j - 1] + rc[m - j - 1];
+                if (v < best) { best = v; s = j; }
+            }
+            cost[m - 1] = best;
+            split[m - 1] = (uint8_t)s;
+        }
+        cost[0] = a + cost[7];
+#pragma unroll
+        for (int m = 2; m < 8; ++m)
+            if (cost[0] <= cost[m - 1]) { cost[m - 1] = cost[0]; split[m - 1] = 0; }
+    }
+    for (int m = 0; m < 7; ++m) out[m] = cost[m];
+    uint32_t w[2] = {0u, 0u};
+    for (int m = 0; m < 8; ++m) w[m >> 2] |= (uint32_t)split[m] << (8 * (m & 3));
+    *reinterpret_cast<uint2*>(f.split + 8ll * k) = make_uint2(w[0], w[1]);
+}
 
 struct PlocArrays {
     const int* sorted;      // primitives by (segment, Morton code)
@@ -458,6 +498,7 @@ __global__ void __launch_bounds__(kBlock) ploc_kernel(Forest f, PlocArrays p, Bu
             f.cnt[k] = c;
             f.cost[k] = lf ? leaf : inner;
             f.leafy[k] = lf ? 1 : 0;
+            choose_collapse(f, k, l, r, lf, a);
             cl2[to] = f.n + k;
             box2[to] = b;
         }
@@ -612,9 +653,10 @@ struct CollapseArrays {
     int* mesh_root;         // wide root per mesh of the scene (this batch's meshes are written)
 };
 
-// The children of queue entry e (whole warp, eight lanes per entry): lane i of the octet returns
-// child i or -1.
-__device__ __forceinline__ int gather_children(const Forest& f, int node) {
+// The children of a top-level wide node (whole warp, eight lanes per node, node < 0: none): lane i
+// returns child i or -1. The internal child of largest area is opened until there are eight (as
+// the host converter does at the top level).
+__device__ __forceinline__ int gather_largest(const Forest& f, int node) {
     const unsigned full = 0xffffffffu;
     const int i = threadIdx.x & 7;
     int kid = -1, nk = 0;
@@ -629,7 +671,6 @@ __device__ __forceinline__ int gather_children(const Forest& f, int node) {
     }
     float area = kid >= 0 && !is_leafy(f, kid) ? half_area(f.nbox[kid]) : -1.0f;
     for (int round = 0; round < 6; ++round) {
-        // The internal child of largest area, the first of equals.
         float ba = area;
         int bi = i;
         for (int o = 4; o > 0; o >>= 1) {
@@ -650,6 +691,34 @@ __device__ __forceinline__ int gather_children(const Forest& f, int node) {
         }
         ++nk;
         if (i >= nk) { kid = -1; area = -1.0f; }
+    }
+    return kid;
+}
+
+// The children of wide node `node` (whole warp, eight lanes per node, node < 0: none): a lane
+// returns a child or -1. An entry (binary node, m) stands at the first of the m lanes it may
+// fill and hands the right child's share to the lane where that begins.
+__device__ __forceinline__ int gather_children(const Forest& f, int node) {
+    const unsigned full = 0xffffffffu;
+    const int i = threadIdx.x & 7;
+    int kid = i == 0 ? node : -1, m = i == 0 && node >= 0 ? 8 : 0;
+    bool open = m > 0 && !is_leafy(f, node);     // the wide node itself is opened in any case
+    while (__ballot_sync(full, open) != 0u) {
+        int k = 0, right = -1;
+        if (open) {
+            k = f.split[8ll * (kid - f.n) + m - 1];
+            right = f.right[kid - f.n];
+            kid = f.left[kid - f.n];
+        }
+        const int take = open ? i + k : -1, share = m - k;
+        // Each lane looks for the opened entry that hands over to it.
+        int from = -1;
+        for (int s = 0; s < 8; ++s)
+            if (__shfl_sync(full, take, s, 8) == i) from = s;
+        const int r = __shfl_sync(full, right, from & 7, 8), rm = __shfl_sync(full, share, from & 7, 8);
+        if (open) m = k;
+        if (from >= 0) { kid = r; m = rm; }
+        open = (open || from >= 0) && !is_leafy(f, kid) && m > 1 && f.split[8ll * (kid - f.n) + m - 1] != 0;
     }
     return kid;
 }
@@ -782,7 +851,8 @@ __global__ void __launch_bounds__(kBlock) collapse_kernel(Forest f, CollapseArra
             for (int g = e0; g < e1; g += kGroup) {
                 const int e = g + oct;
                 const bool has = e < e1;
-                const int kid = gather_children(f, has ? queue[e] : -1);
+                const int node = has ? queue[e] : -1;
+                const int kid = part == 0 ? gather_children(f, node) : gather_largest(f, node);
                 const bool lf = kid >= 0 && is_leafy(f, kid);
                 const int ni = __popc(octet_ballot(kid >= 0 && !lf));
                 int np = lf ? prim_count(f, kid) : 0;
@@ -886,8 +956,8 @@ struct BuildArrays {
     Box6 *boxes, *nbox, *clbox[2];
     uint64_t* keys[2];
     int *vals[2], *cl[2], *sg[2], *link, *left, *right, *cnt;
-    float* cost;
-    uint8_t* leafy;
+    float *cost, *area;
+    uint8_t *leafy, *split;
     int *roots, *queue[2], *kids, *n_int, *n_prims;
     int2* sums;
     void* temp;
@@ -907,6 +977,7 @@ struct BuildArrays {
             s.take(queue[k], n);
         }
         s.take(link, n); s.take(left, n); s.take(right, n); s.take(cnt, n); s.take(cost, n); s.take(leafy, n);
+        s.take(area, 7 * n); s.take(split, 8 * n);
         s.take(roots, max_seg);
         s.take(kids, 8 * n); s.take(n_int, n); s.take(n_prims, n);
         s.take(sums, kMaxBuildBlocks);
@@ -1066,7 +1137,8 @@ int build_scene_gpu(const imbart_mesh_desc* meshes, int n_meshes, const imbart_i
                ck(cub::DeviceRadixSort::SortPairs(A.temp, temp_bytes, A.keys[0], A.keys[1], A.vals[0], A.vals[1], n, 0,
                                                   3 * bits + seg_bits, st), "SortPairs");
         if (!good) break;
-        Forest f{n, n_seg, top_seg, A.seg_first, A.nbox, A.left, A.right, A.cnt, A.cost, A.leafy, A.roots};
+        Forest f{n, n_seg, top_seg, A.seg_first, A.nbox, A.left, A.right, A.cnt, A.cost, A.leafy, A.area, A.split,
+                 A.roots};
         PlocArrays p{};
         p.sorted = A.vals[1];
         p.boxes = A.boxes;
