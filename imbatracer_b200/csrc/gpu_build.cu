@@ -39,8 +39,11 @@
 #include <chrono>
 #include <climits>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
+#include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "imbart_internal.h"
@@ -250,14 +253,18 @@ __global__ void morton_kernel(const Box6* __restrict__ boxes, int n, const int* 
 
 // ---------------------------------------------------------------------------------------
 // Barrier of a cooperative launch's blocks. Every block passes the same barriers in the same
-// order; thread 0's fences order the block's accesses before and after it. The wait gives up
-// after kSpinLimit polls and sets *error, which every block reads after the barrier and then
-// leaves by.
+// order; thread 0's fences order the block's accesses before and after it. The last block to
+// arrive opens the barrier for the others, which poll a word of its own, so that their polls do
+// not hold up the arrivals. A wait gives up after kSpinLimit polls and sets *error, which every
+// block reads after the barrier and then leaves by.
 // ---------------------------------------------------------------------------------------
-constexpr int kSpinLimit = 1 << 24;
+constexpr int kSpinLimit = 1 << 22;
 
 struct BuildState {
     unsigned arrived;       // barrier: blocks arrived so far
+    unsigned pad0[31];
+    unsigned open;          // arrivals of the barriers passed so far
+    unsigned pad1[31];
     int error;
     int wide_count;         // wide nodes written
     int bottom_nodes;       // of these, mesh trees
@@ -271,10 +278,14 @@ __device__ __forceinline__ bool grid_barrier(BuildState* st, unsigned& target) {
     if (threadIdx.x == 0) {
         target += gridDim.x;
         __threadfence();
-        atomicAdd(&st->arrived, 1u);
-        int polls = 0;
-        while ((int)(*(volatile unsigned*)&st->arrived - target) < 0) {
-            if (++polls > kSpinLimit) { atomicExch(&st->error, kErrBarrier); break; }
+        if (atomicAdd(&st->arrived, 1u) + 1u == target) {
+            atomicExch(&st->open, target);
+        } else {
+            int polls = 0;
+            while ((int)(*(volatile unsigned*)&st->open - target) < 0) {
+                if (++polls > kSpinLimit) { atomicExch(&st->error, kErrBarrier); break; }
+                __nanosleep(20);
+            }
         }
         __threadfence();
         s_error = *(volatile int*)&st->error;
@@ -373,18 +384,21 @@ struct PlocArrays {
     int2* sums;             // per block
 };
 constexpr int kKeep = -1, kGone = -2;
-constexpr int kSolo = 2048; // clusters from which one block goes on alone (no barriers)
+constexpr int kSolo = 1024; // clusters from which one block goes on alone (no barriers)
+constexpr int kOwn = kBlock - 2 * kRadius;   // clusters of a tile: its neighbours within kRadius fill the block
 
-// 3. PLOC. Each block owns a contiguous run of clusters and takes it tile by tile: boxes of the
+// 3. PLOC. Each block owns a contiguous run of clusters and takes it in tiles of kOwn: boxes of the
 // tile and 32 positions on either side in shared memory, nearest neighbours of the tile and 16
-// positions on either side (so that a merge is known to be mutual without another barrier), then
+// positions on either side, one per thread (so that a merge is known to be mutual without another
+// barrier), then
 // after a barrier the compaction into the other buffers at the blocks' scanned offsets. Two
 // barriers a round; below kSolo clusters one block goes on alone.
 __global__ void __launch_bounds__(kBlock) ploc_kernel(Forest f, PlocArrays p, BuildState* st) {
     constexpr int kHalo = 2 * kRadius;
-    __shared__ Box6 sb[kBlock + 2 * kHalo];
-    __shared__ int ss[kBlock + 2 * kHalo];
-    __shared__ int snn[kBlock + 2 * kRadius];
+    __shared__ float4 sb4[kOwn + 2 * kHalo];     // staged boxes: low corner, high x
+    __shared__ float2 sb2[kOwn + 2 * kHalo];     // high y, z
+    __shared__ int ss[kOwn + 2 * kHalo];
+    __shared__ int snn[kBlock];
     __shared__ int wk[kBlock / 32], wm[kBlock / 32];
     if (*(volatile int*)&st->error != 0) return;
     unsigned target = 0;
@@ -406,46 +420,58 @@ __global__ void __launch_bounds__(kBlock) ploc_kernel(Forest f, PlocArrays p, Bu
             solo = true;
         }
         const int blocks = solo ? 1 : gridDim.x;
-        const int chunk = ((m + blocks - 1) / blocks + kBlock - 1) / kBlock * kBlock;
+        const int chunk = ((m + blocks - 1) / blocks + kOwn - 1) / kOwn * kOwn;
         const int lo = min((solo ? 0 : blockIdx.x) * chunk, m), hi = min(lo + chunk, m);
         const int* cl = p.cl[cur];
         const int* sg = p.sg[cur];
         const Box6* box = p.box[cur];
         int kept = 0, merged = 0;
-        for (int tile = lo; tile < hi; tile += kBlock) {
+        for (int tile = lo; tile < hi; tile += kOwn) {
             const int first = tile - kHalo;
             __syncthreads();
-            for (int t = tid; t < kBlock + 2 * kHalo; t += kBlock) {
+            for (int t = tid; t < kOwn + 2 * kHalo; t += kBlock) {
                 const int j = first + t;
                 ss[t] = -1;
-                if (j >= 0 && j < m) { sb[t] = box[j]; ss[t] = sg[j]; }
-            }
-            __syncthreads();
-            for (int t = tid; t < kBlock + 2 * kRadius; t += kBlock) {
-                const int c = t + kRadius;   // position in the staged run
-                int bj = -1;
-                if (ss[c] >= 0) {
-                    const Box6 bi = sb[c];
-                    const int seg = ss[c];
-                    float best = FLT_MAX;
-                    for (int j = c - kRadius; j <= c + kRadius; ++j) {
-                        if (j == c || ss[j] != seg) continue;
-                        const float d = half_area(merge(bi, sb[j]));
-                        if (d < best) { best = d; bj = j; }   // ties: the smaller position
-                    }
+                if (j >= 0 && j < m) {
+                    const Box6 b = box[j];
+                    sb4[t] = make_float4(b.lo[0], b.lo[1], b.lo[2], b.hi[0]);
+                    sb2[t] = make_float2(b.hi[1], b.hi[2]);
+                    ss[t] = sg[j];
                 }
-                snn[t] = bj;
             }
             __syncthreads();
-            const int i = tile + tid;
-            if (i < hi) {
-                const int c = tid + kHalo, j = snn[tid + kRadius];
-                const bool mutual = j >= 0 && snn[j - kRadius] == c;
-                p.link[i] = !mutual ? kKeep : c < j ? first + j : kGone;
-                merged += mutual && c < j ? 1 : 0;
-                kept += mutual && c > j ? 0 : 1;
+            // Thread t finds the nearest neighbour of staged position t + kRadius.
+            const int c = tid + kRadius;
+            const int seg = ss[c];
+            int bj = -1;
+            if (seg >= 0) {
+                const float4 a4 = sb4[c];
+                const float2 a2 = sb2[c];
+                float best = FLT_MAX;
+#pragma unroll 8
+                for (int o = 0; o < 2 * kRadius; ++o) {
+                    const int j = c + (o < kRadius ? o - kRadius : o - kRadius + 1);
+                    const float4 b4 = sb4[j];
+                    const float2 b2 = sb2[j];
+                    // half_area of the union
+                    const float dx = fmaxf(fmaxf(a4.w, b4.w) - fminf(a4.x, b4.x), 0.0f);
+                    const float dy = fmaxf(fmaxf(a2.x, b2.x) - fminf(a4.y, b4.y), 0.0f);
+                    const float dz = fmaxf(fmaxf(a2.y, b2.y) - fminf(a4.z, b4.z), 0.0f);
+                    const float d = ss[j] == seg ? dx * (dy + dz) + dy * dz : FLT_MAX;
+                    if (d < best) { best = d; bj = j; }   // ties: the smaller position
+                }
+            }
+            snn[tid] = bj;
+            __syncthreads();
+            const int i = tile + tid - kRadius;
+            if (tid >= kRadius && tid < kRadius + kOwn && i < hi) {
+                const bool mutual = bj >= 0 && snn[bj - kRadius] == c;
+                p.link[i] = !mutual ? kKeep : c < bj ? first + bj : kGone;
+                merged += mutual && c < bj ? 1 : 0;
+                kept += mutual && c > bj ? 0 : 1;
             }
         }
+        __syncthreads();    // the links below are read by other threads of the block
         const int2 mine = block_sum(kept, merged);
         int2 before = make_int2(0, 0), total = mine;
         if (!solo) {
@@ -937,6 +963,50 @@ struct Slab {
     }
 };
 
+// The builds' scratch is kept between them, one allocation per device and at most kKeptScratch
+// bytes of it; a scene's records share one allocation too. An allocation and its release cost
+// 0.6 ms here whatever the size: the instanced scene's build took 2.8 ms with five of them (and
+// with PLOC tiles of two passes and barriers polled where they count arrivals), 1.6 ms. A build
+// takes the kept one, so concurrent builds have their own, and hands it back after its stream is
+// done; imbart_invalidate_scenes frees it.
+constexpr size_t kKeptScratch = 256ull << 20;
+struct KeptScratch {
+    char* base = nullptr;
+    size_t bytes = 0;
+};
+std::mutex g_scratch_mutex;
+KeptScratch g_scratch[64];
+
+char* take_scratch(int device, size_t& bytes) {
+    if (device >= 0 && device < 64) {
+        std::lock_guard<std::mutex> lk(g_scratch_mutex);
+        KeptScratch& k = g_scratch[device];
+        if (k.base && k.bytes >= bytes) {
+            char* p = k.base;
+            bytes = k.bytes;
+            k = KeptScratch{};
+            return p;
+        }
+    }
+    char* p = nullptr;
+    if (cudaMalloc((void**)&p, bytes) == cudaSuccess) return p;
+    (void)cudaGetLastError();
+    release_build_scratch();
+    return dmalloc(&p, bytes) ? p : nullptr;
+}
+
+void give_scratch(int device, char* base, size_t bytes) {
+    if (base && device >= 0 && device < 64 && bytes <= kKeptScratch) {
+        std::lock_guard<std::mutex> lk(g_scratch_mutex);
+        KeptScratch& k = g_scratch[device];
+        if (k.bytes < bytes) {
+            std::swap(k.base, base);
+            k.bytes = bytes;
+        }
+    }
+    cudaFree(base);
+}
+
 constexpr long long kBatchPrims = 32ll << 20;   // meshes are built together up to this many primitives
 constexpr int kMaxBuildBlocks = 2048;
 
@@ -961,10 +1031,13 @@ struct BuildArrays {
     int *roots, *queue[2], *kids, *n_int, *n_prims;
     int2* sums;
     void* temp;
-    WideNode* nodes;        // the batch's wide nodes when it is the only one
+    // the scene's records when there is one batch: they move to an allocation of their size
+    WideNode* nodes;
+    WideTri* tris;
+    WideInst* winsts;
 
     void layout(Slab& s, long long verts_n, int n_meshes, int n_insts, size_t n, int max_seg, size_t temp_bytes,
-                size_t nodes_n) {
+                size_t nodes_n, size_t tris_n, size_t insts_n) {
         s.take(verts, 3 * (size_t)verts_n);
         s.take(vert_first, n_meshes); s.take(vert_count, n_meshes); s.take(tri_offset, n_meshes);
         s.take(mesh_root, n_meshes);
@@ -984,7 +1057,7 @@ struct BuildArrays {
         char* t = nullptr;
         s.take(t, temp_bytes);
         temp = t;
-        s.take(nodes, nodes_n);
+        s.take(nodes, nodes_n); s.take(tris, tris_n); s.take(winsts, insts_n);
     }
 };
 
@@ -1062,7 +1135,7 @@ int build_scene_gpu(const imbart_mesh_desc* meshes, int n_meshes, const imbart_i
     batch_end.push_back(n_meshes);
     cap = std::max(cap, in_batch + n_insts);
     max_seg = std::max(max_seg, n_meshes - batch_first + 1);
-    const bool single = batch_end.size() == 1;
+    const bool single = batch_end.size() == 1 && cap <= kBatchPrims;
     int prev = 0;
     cudaGetDevice(&prev);
     if (!ck(cudaSetDevice(device), "cudaSetDevice")) return IMBART_ERR_CUDA;
@@ -1075,21 +1148,29 @@ int build_scene_gpu(const imbart_mesh_desc* meshes, int n_meshes, const imbart_i
                                     (const int*)nullptr, (int*)nullptr, (int)cap, 0, 64);
     Slab slab;
     BuildArrays A{};
-    A.layout(slab, total_verts, n_meshes, n_insts, (size_t)cap, max_seg, temp_bytes, single ? node_cap : 0);
-    char* base = nullptr;
+    auto layout = [&] {
+        slab.used = 0;
+        A.layout(slab, total_verts, n_meshes, n_insts, (size_t)cap, max_seg, temp_bytes, single ? node_cap : 0,
+                 single ? (size_t)total_tris : 0, single ? (size_t)n_insts : 0);
+    };
+    layout();
+    size_t scratch_bytes = slab.used;
+    char* base = take_scratch(device, scratch_bytes);
     WideNode* nodes = nullptr;
     WideTri* tris = nullptr;
     WideInst* winsts = nullptr;
-    bool good = dmalloc(&base, slab.used) && dmalloc(&tris, total_tris) && dmalloc(&winsts, n_insts) &&
-                (single || dmalloc(&nodes, node_cap));
+    int* error_flags = nullptr;
+    char* block = nullptr;
+    bool good = base && (single || (dmalloc(&nodes, node_cap) && dmalloc(&tris, total_tris) &&
+                                    dmalloc(&winsts, n_insts) && dmalloc(&error_flags, 4)));
     auto copy = [&](void* dst, const void* src, size_t bytes, cudaMemcpyKind kind) {
         return ck(cudaMemcpyAsync(dst, src, bytes, kind, st), "cudaMemcpyAsync");
     };
     BuildState hs{};
     if (good) {
-        slab.used = 0;
         slab.base = base;
-        A.layout(slab, total_verts, n_meshes, n_insts, (size_t)cap, max_seg, temp_bytes, single ? node_cap : 0);
+        layout();
+        if (single) { nodes = A.nodes; tris = A.tris; winsts = A.winsts; }
         good = copy(A.vert_first, vert_first.data(), sizeof(long long) * n_meshes, cudaMemcpyHostToDevice) &&
                copy(A.vert_count, vert_count.data(), sizeof(int) * n_meshes, cudaMemcpyHostToDevice) &&
                copy(A.tri_offset, tri_offset.data(), sizeof(int) * n_meshes, cudaMemcpyHostToDevice) &&
@@ -1115,7 +1196,7 @@ int build_scene_gpu(const imbart_mesh_desc* meshes, int n_meshes, const imbart_i
         int seg_bits = 0;
         while ((1ll << seg_bits) < n_seg) ++seg_bits;
         const int bits = std::min(21, (64 - seg_bits) / 3);
-        hs.arrived = 0;
+        hs.arrived = hs.open = 0;
         hs.error = 0;
         good = good && copy(A.seg_first, seg_first.data(), sizeof(int) * (n_seg + 1), cudaMemcpyHostToDevice) &&
                copy(A.state, &hs, sizeof(hs), cudaMemcpyHostToDevice);
@@ -1148,14 +1229,14 @@ int build_scene_gpu(const imbart_mesh_desc* meshes, int n_meshes, const imbart_i
         BuildState* state = A.state;
         void* pargs[] = {&f, &p, &state};
         good = ck(cudaLaunchCooperativeKernel((const void*)ploc_kernel,
-                                              dim3(coop_blocks((const void*)ploc_kernel, device, n, kBlock)),
+                                              dim3(coop_blocks((const void*)ploc_kernel, device, n, kOwn)),
                                               dim3(kBlock), pargs, 0, st), "clustering launch") &&
-               ck(cudaMemsetAsync(&A.state->arrived, 0, sizeof(unsigned), st), "cudaMemsetAsync");
+               ck(cudaMemsetAsync(A.state, 0, offsetof(BuildState, error), st), "cudaMemsetAsync");
         if (!good) break;
         CollapseArrays c{{A.queue[0], A.queue[1]}, A.kids, A.n_int, A.n_prims, A.sums, A.mesh_root};
         LeafOut lo{n_tris, A.verts, A.idx, A.seg_first, n_seg, A.vert_first + k0, A.tri_offset + k0, tris, A.insts,
                    A.mesh_root, winsts};
-        WideNode* wn = single ? A.nodes : nodes;
+        WideNode* wn = nodes;
         int wide_first = hs.wide_count, tri_first = hs.tri_count, first_mesh = k0;
         void* cargs[] = {&f, &c, &wn, &wide_first, &tri_first, &first_mesh, &lo, &state};
         good = ck(cudaLaunchCooperativeKernel((const void*)collapse_kernel,
@@ -1169,11 +1250,31 @@ int build_scene_gpu(const imbart_mesh_desc* meshes, int n_meshes, const imbart_i
             good = false;
         }
     }
-    if (good && single)
-        good = dmalloc(&nodes, hs.wide_count) &&
-               copy(nodes, A.nodes, sizeof(WideNode) * (size_t)hs.wide_count, cudaMemcpyDeviceToDevice) &&
+    if (good && single) {
+        // The records into one allocation of their size, error flags last.
+        Slab out;
+        auto place = [&] {
+            out.used = 0;
+            out.take(nodes, hs.wide_count);
+            out.take(tris, hs.tri_count);
+            out.take(winsts, n_insts);
+            out.take(error_flags, 4);
+        };
+        place();
+        good = dmalloc(&block, out.used);
+        if (good) {
+            out.base = block;
+            place();
+            good = copy(nodes, A.nodes, sizeof(WideNode) * (size_t)hs.wide_count, cudaMemcpyDeviceToDevice) &&
+                   copy(tris, A.tris, sizeof(WideTri) * (size_t)hs.tri_count, cudaMemcpyDeviceToDevice) &&
+                   copy(winsts, A.winsts, sizeof(WideInst) * (size_t)n_insts, cudaMemcpyDeviceToDevice);
+        }
+    }
+    if (good)
+        good = ck(cudaMemsetAsync(error_flags, 0, 4 * sizeof(int), st), "cudaMemsetAsync") &&
                ck(cudaStreamSynchronize(st), "cudaStreamSynchronize");
-    cudaFree(base);
+    if (!good) cudaStreamSynchronize(st);   // nothing of a failed build still runs on the scratch
+    give_scratch(device, base, scratch_bytes);
     if (good) {
         int direct_inst = -1;
         WideInst w{};
@@ -1182,19 +1283,14 @@ int build_scene_gpu(const imbart_mesh_desc* meshes, int n_meshes, const imbart_i
         // The meshes' roots are the first nodes of their batch.
         int direct_root = -1;
         if (direct_inst >= 0 && n_meshes == 1) direct_root = 0;
-        imbart_scene* s = scene_adopt_device_arrays(device, nodes, hs.wide_count, hs.wide_count - hs.bottom_nodes, tris,
-                                                    hs.tri_count, winsts, n_insts, hs.bottom_nodes, direct_root,
-                                                    direct_inst);
-        if (s) {
-            *out = s;
-            if (build_ms)
-                *build_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
-        } else {
-            good = false;
-        }
-    }
-    if (!good) {
-        cudaFree(nodes); cudaFree(tris); cudaFree(winsts);
+        *out = scene_adopt_device_arrays(device, block, nodes, hs.wide_count, hs.wide_count - hs.bottom_nodes, tris,
+                                         hs.tri_count, winsts, n_insts, error_flags, hs.bottom_nodes, direct_root,
+                                         direct_inst);
+        if (build_ms)
+            *build_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    } else {
+        cudaFree(block);
+        if (!single) { cudaFree(nodes); cudaFree(tris); cudaFree(winsts); cudaFree(error_flags); }
         if (!rc) rc = imbart_last_error() ? imbart_last_error() : IMBART_ERR_CUDA;
     }
     cudaSetDevice(prev);
@@ -1454,6 +1550,20 @@ int refit_scene(imbart_scene* scene, const float* verts, long long n_verts, cons
 }
 
 }  // namespace
+
+void release_build_scratch() {
+    std::lock_guard<std::mutex> lk(g_scratch_mutex);
+    int prev = 0;
+    cudaGetDevice(&prev);
+    for (int d = 0; d < 64; ++d) {
+        if (!g_scratch[d].base) continue;
+        cudaSetDevice(d);
+        cudaFree(g_scratch[d].base);
+        g_scratch[d] = KeptScratch{};
+    }
+    cudaSetDevice(prev);
+}
+
 }  // namespace imbart
 
 extern "C" int imbart_scene_refit(imbart_scene* scene, const float* vertices, long long n_vertices,

@@ -151,12 +151,15 @@ void scene_pool_view_destroy(imbart_scene* s);
 // identity instance (direct_root -1: none).
 void scene_pool_view_set_root(imbart_scene* s, int root, int direct_root = -1, int direct_inst = -1);
 
-// A scene over device arrays built on the GPU; the scene takes ownership (cudaFree on
-// destroy). NULL on error (the arrays are then still the caller's). direct_root / direct_inst:
-// mesh root and id of a top level that is one identity instance (-1: none).
-imbart_scene* scene_adopt_device_arrays(int device, WideNode* nodes, int64_t n_nodes, int64_t top_nodes,
-                                        WideTri* tris, int64_t n_tris, WideInst* insts, int64_t n_insts, int root,
-                                        int direct_root, int direct_inst);
+// A scene over device arrays built on the GPU, which it takes over: all in one allocation
+// `block` (error_flags, 4 zeroed ints, among them), or allocations of their own (block NULL).
+// direct_root / direct_inst: mesh root and id of a top level that is one identity instance
+// (-1: none).
+imbart_scene* scene_adopt_device_arrays(int device, void* block, WideNode* nodes, int64_t n_nodes, int64_t top_nodes,
+                                        WideTri* tris, int64_t n_tris, WideInst* insts, int64_t n_insts,
+                                        int* error_flags, int root, int direct_root, int direct_inst);
+// Frees the scratch that device builds keep between calls (gpu_build.cu).
+void release_build_scratch();
 
 // Device scratch of `bytes` for a scene's refits, allocated by the first call and freed with the
 // scene (*fresh: this call allocated it). NULL on error. bytes = 0 frees it.

@@ -108,7 +108,9 @@ void occluded_cpu_masked_instanced(int root, imbart_node4* nodes, imbart_instanc
                                    char* mask_buffer, int count);
 
 /* Drops every scene the drop-in entry points converted and cached. Call after rewriting
- * node, triangle or instance buffers in place (Scene::upload_top_level_accel, scene.cpp:167-188). */
+ * node, triangle or instance buffers in place (Scene::upload_top_level_accel, scene.cpp:167-188).
+ * Also frees the scratch that imbart_scene_build_gpu keeps between calls (at most 256 MiB per
+ * device). */
 void imbart_invalidate_scenes(void);
 
 /* ------------------------------------------------------------------------------------ */
