@@ -135,25 +135,25 @@ __device__ __forceinline__ int knn_keep(KnnScratch<kCap>& s, int n, int k, bool 
     constexpr unsigned kFull = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int per = (n + 31) >> 5;
-    for (int j = n + lane; j < ((n + 3) & ~3); j += 32) s.d2[j] = 0xffffffffu;
+    if (lane < (-n & 3)) s.d2[n + lane] = 0xffffffffu;    // to a multiple of four
     __syncwarp();
     uint32_t d[kPer];
     int id[kPer], rank[kPer];
     int sum = 0;
 #pragma unroll
     for (int t = 0; t < kPer; ++t) {
-        const bool has = 32 * t + lane < n;
-        d[t] = has ? s.d2[32 * t + lane] : 0u;
-        id[t] = has ? s.id[32 * t + lane] : 0;
-        rank[t] = 0;
-        if (t < per) {
-            for (int j = 0; j < n; j += 4) {
-                const uint4 o = *reinterpret_cast<const uint4*>(s.d2 + j);
-                rank[t] += (o.x <= d[t]) + (o.y <= d[t]) + (o.z <= d[t]) + (o.w <= d[t]);
-            }
-            rank[t] -= 1;
-            if (has) sum += rank[t];
+        if (t > 0 && t >= per) { d[t] = 0u; id[t] = 0; rank[t] = kCap; continue; }
+        const int i = 32 * t + lane;
+        d[t] = s.d2[i];        // beyond n: left over, not used
+        id[t] = s.id[i];
+        int r = -1;
+#pragma unroll 2
+        for (int j = 0; j < n; j += 4) {
+            const uint4 o = *reinterpret_cast<const uint4*>(s.d2 + j);
+            r += (o.x <= d[t]) + (o.y <= d[t]) + (o.z <= d[t]) + (o.w <= d[t]);
         }
+        rank[t] = r;
+        if (i < n) sum += r;
     }
     int kept = n;
     const bool ties = __reduce_add_sync(kFull, sum) != n * (n - 1) / 2;
