@@ -756,13 +756,6 @@ bool grow(T** p, long long* cap, long long need, long long keep = 0) {
     return true;
 }
 
-template <typename T>
-bool realloc_exact(T** ptr, size_t elems) {
-    cudaFree(*ptr);
-    *ptr = nullptr;
-    return ok(cudaMalloc((void**)ptr, std::max<size_t>(elems, 1) * sizeof(T)), "cudaMalloc");
-}
-
 }  // namespace
 }  // namespace imbart
 
@@ -770,6 +763,7 @@ namespace imbart {
 namespace {
 // Scratch of the pixel-size estimate: camera, probe rays and hits, per-query distances.
 struct PixelProbe {
+    void* block = nullptr;          // the arrays below
     float* cam = nullptr;
     float4* rays = nullptr;
     int4* hits = nullptr;
@@ -777,8 +771,8 @@ struct PixelProbe {
     long long cap = 0;
     std::vector<float4> host;
     void release() {
-        cudaFree(cam); cudaFree(rays); cudaFree(hits); cudaFree(dist);
-        cam = nullptr; rays = nullptr; hits = nullptr; dist = nullptr; cap = 0;
+        cudaFree(block);
+        block = nullptr; cam = nullptr; rays = nullptr; hits = nullptr; dist = nullptr; cap = 0;
     }
 };
 }  // namespace
@@ -801,6 +795,7 @@ struct imbart_vcm {
     imbart::PixelProbe probe;
     int device = 0;
     // light-path slots
+    void* l_block = nullptr;        // the arrays up to bsums
     long long l_cap = 0;
     float4* l_rays = nullptr;
     int4* l_hits = nullptr;
@@ -824,6 +819,7 @@ struct imbart_vcm {
     imbart_hashgrid* grid = nullptr;
     bool grid_built = false;
     // camera queues
+    void* c_block = nullptr;        // the arrays up to c_merge
     long long c_cap = 0;
     float4* c_rays[2] = {nullptr, nullptr};
     int* c_pixel[2] = {nullptr, nullptr};
@@ -833,6 +829,7 @@ struct imbart_vcm {
     int4* c_hits = nullptr;
     float4* c_merge = nullptr;      // queued camera vertices for merging (7 float4 each)
     // Material grouping of a wavefront (keys, shading order, 8 counts then offsets per tile).
+    void* sort_block = nullptr;
     long long sort_cap = 0;
     bool use_perm = false;
     uint8_t* keys = nullptr;
@@ -840,6 +837,7 @@ struct imbart_vcm {
     int* tile_counts = nullptr;
     // Two shadow queues: a wavefront's shadow rays are traced and accumulated on a stream of
     // their own beside the next wavefront (begin_wave / trace_shadows).
+    void* s_block = nullptr;
     long long s_cap = 0;
     imbart::ShadowQueue queue[2];
     cudaStream_t side = nullptr;
@@ -855,22 +853,12 @@ namespace imbart {
 namespace {
 
 void free_vcm(imbart_vcm* v) {
-    void* ptrs[] = {v->keys, v->perm, v->tile_counts,
-                    v->l_rays, v->l_hits, v->l_rng, v->l_thr, v->l_w, v->l_rays2, v->l_rng2, v->l_thr2, v->l_w2,
-                    v->stage, v->vflags, v->bsums, v->d_tiles,
-                    v->cache, v->c_hits, v->c_merge, v->counts};
+    void* ptrs[] = {v->l_block, v->c_block, v->s_block, v->sort_block, v->d_tiles, v->cache, v->counts};
     for (void* p : ptrs) cudaFree(p);
-    for (ShadowQueue& q : v->queue) {
-        void* qp[] = {q.rays, q.hits, q.pixel, q.contrib};
-        for (void* p : qp) cudaFree(p);
+    for (ShadowQueue& q : v->queue)
         if (q.done) cudaEventDestroy(q.done);
-    }
     if (v->shaded) cudaEventDestroy(v->shaded);
     if (v->side) cudaStreamDestroy(v->side);
-    for (int k = 0; k < 2; ++k) {
-        void* q[] = {v->c_rays[k], v->c_pixel[k], v->c_rng[k], v->c_thr[k], v->c_w[k]};
-        for (void* p : q) cudaFree(p);
-    }
     cudaFreeHost(v->host_counts);
     if (v->grid) imbart_hashgrid_destroy(v->grid);
     v->probe.release();
@@ -887,10 +875,15 @@ bool valid_settings(const imbart_vcm_settings* st) {
 bool ensure_shadow(imbart_vcm* v, long long need) {
     if (v->s_cap >= need) return true;
     need = std::max(need, v->s_cap * 3 / 2);   // geometric growth: reallocation synchronizes the device
-    bool good = true;
-    for (ShadowQueue& q : v->queue)
-        good = good && realloc_exact(&q.rays, 2 * (size_t)need) && realloc_exact(&q.hits, (size_t)need) &&
-               realloc_exact(&q.pixel, (size_t)need) && realloc_exact(&q.contrib, (size_t)need);
+    const size_t c = (size_t)need;
+    const bool good = ok(realloc_block(&v->s_block, [&](BlockLayout& at) {
+        for (ShadowQueue& q : v->queue) {
+            at(&q.rays, 2 * c);
+            at(&q.hits, c);
+            at(&q.pixel, c);
+            at(&q.contrib, c);
+        }
+    }), "cudaMalloc");
     v->s_cap = good ? need : 0;
     return good;
 }
@@ -945,8 +938,11 @@ bool group_paths(imbart_vcm* v, const imbart_shading* sh, int n, cudaStream_t s,
     if (!v->use_perm) return true;
     if (v->sort_cap < n) {
         const long long c = std::max<long long>(n, v->sort_cap * 3 / 2);
-        const bool good = realloc_exact(&v->keys, (size_t)c) && realloc_exact(&v->perm, (size_t)c) &&
-                          realloc_exact(&v->tile_counts, (size_t)pt::kShadeKeys * pt::group_tiles(c));
+        const bool good = ok(realloc_block(&v->sort_block, [&](BlockLayout& at) {
+            at(&v->keys, (size_t)c);
+            at(&v->perm, (size_t)c);
+            at(&v->tile_counts, (size_t)pt::kShadeKeys * pt::group_tiles(c));
+        }), "cudaMalloc");
         v->sort_cap = good ? c : 0;
         if (!good) return false;
     }
@@ -1038,11 +1034,14 @@ int estimate_pixel_size(const imbart_scene* scene, const imbart_camera* cam, flo
     }
     const int nx = (cam->width + 7) / 8, ny = (cam->height + 7) / 8, nq = nx * ny;
     bool good = true;
-    if (!pb.cam) good = ok(cudaMalloc((void**)&pb.cam, sizeof(float) * 19), "cudaMalloc");
-    if (good && pb.cap < nq) {
+    if (pb.cap < nq) {
         const long long c = std::max<long long>(nq, pb.cap * 3 / 2);
-        good = realloc_exact(&pb.rays, 8 * (size_t)c) && realloc_exact(&pb.hits, 4 * (size_t)c) &&
-               realloc_exact(&pb.dist, (size_t)c);
+        good = ok(realloc_block(&pb.block, [&](BlockLayout& at) {
+            at(&pb.cam, 19);
+            at(&pb.rays, 8 * (size_t)c);
+            at(&pb.hits, 4 * (size_t)c);
+            at(&pb.dist, (size_t)c);
+        }), "cudaMalloc");
         pb.cap = good ? c : 0;
     }
     pb.host.resize(nq);
@@ -1186,16 +1185,26 @@ int imbart_vcm_light_pass_range(imbart_vcm* v, const imbart_scene* scene, const 
     if (v->l_cap < P) {
         const long long c = std::max<long long>(P, v->l_cap * 3 / 2);
         const long long cb = (c + kScanTile - 1) / kScanTile;
-        good = realloc_exact(&v->l_rays, 2 * (size_t)c) && realloc_exact(&v->l_hits, (size_t)c) &&
-               realloc_exact(&v->l_rng, (size_t)c) && realloc_exact(&v->l_thr, (size_t)c) &&
-               realloc_exact(&v->l_w, (size_t)c) && realloc_exact(&v->l_rays2, 2 * (size_t)c) &&
-               realloc_exact(&v->l_rng2, (size_t)c) && realloc_exact(&v->l_thr2, (size_t)c) &&
-               realloc_exact(&v->l_w2, (size_t)c) && realloc_exact(&v->stage, 7 * (size_t)c) &&
-               realloc_exact(&v->vflags, (size_t)c) && realloc_exact(&v->bsums, (size_t)cb + 1);
+        good = ok(realloc_block(&v->l_block, [&](BlockLayout& at) {
+            at(&v->l_rays, 2 * (size_t)c);
+            at(&v->l_hits, (size_t)c);
+            at(&v->l_rng, (size_t)c);
+            at(&v->l_thr, (size_t)c);
+            at(&v->l_w, (size_t)c);
+            at(&v->l_rays2, 2 * (size_t)c);
+            at(&v->l_rng2, (size_t)c);
+            at(&v->l_thr2, (size_t)c);
+            at(&v->l_w2, (size_t)c);
+            at(&v->stage, 7 * (size_t)c);
+            at(&v->vflags, (size_t)c);
+            at(&v->bsums, (size_t)cb + 1);
+        }), "cudaMalloc");
         v->l_cap = good ? c : 0;
     }
     if (good && v->tiles_cap < (long long)tiles.size()) {
-        good = realloc_exact(&v->d_tiles, tiles.size());
+        cudaFree(v->d_tiles);
+        v->d_tiles = nullptr;
+        good = ok(cudaMalloc((void**)&v->d_tiles, tiles.size() * sizeof(LightTile)), "cudaMalloc");
         v->tiles_cap = good ? (long long)tiles.size() : 0;
     }
     good = good && ensure_shadow(v, P);
@@ -1239,13 +1248,15 @@ int imbart_vcm_light_pass_range(imbart_vcm* v, const imbart_scene* scene, const 
         n_closest += live;
         ++n_waves;
         // Room for up to n new vertices before the wavefront appends (a larger cache takes over the
-        // vertices once the last append on s is done).
-        if (v->cache_cap < 7ll * (v->cache_count + (long long)n) &&
-            !ok(cudaStreamSynchronize(s), "cudaStreamSynchronize")) {
+        // vertices once the last append on s is done). A new context starts with two per path: light
+        // passes leave 1.5 to 2.
+        long long room = 7ll * (v->cache_count + (long long)n);
+        if (v->cache_cap == 0) room *= 2;
+        if (v->cache_cap < room && !ok(cudaStreamSynchronize(s), "cudaStreamSynchronize")) {
             rc = IMBART_ERR_CUDA;
             break;
         }
-        if (!grow(&v->cache, &v->cache_cap, 7ll * (v->cache_count + (long long)n), 7ll * v->cache_count)) {
+        if (!grow(&v->cache, &v->cache_cap, room, 7ll * v->cache_count)) {
             rc = IMBART_ERR_OUT_OF_MEMORY;
             break;
         }
@@ -1370,11 +1381,17 @@ int imbart_vcm_camera_pass_range(imbart_vcm* v, const imbart_scene* scene, const
     bool good = true;
     if (v->c_cap < chunk) {
         const long long c = std::max(chunk, v->c_cap * 3 / 2);
-        for (int k = 0; k < 2 && good; ++k)
-            good = realloc_exact(&v->c_rays[k], 2 * (size_t)c) && realloc_exact(&v->c_pixel[k], (size_t)c) &&
-                   realloc_exact(&v->c_rng[k], (size_t)c) && realloc_exact(&v->c_thr[k], (size_t)c) &&
-                   realloc_exact(&v->c_w[k], (size_t)c);
-        good = good && realloc_exact(&v->c_hits, (size_t)c) && realloc_exact(&v->c_merge, (size_t)kMergeRec * c);
+        good = ok(realloc_block(&v->c_block, [&](BlockLayout& at) {
+            for (int k = 0; k < 2; ++k) {
+                at(&v->c_rays[k], 2 * (size_t)c);
+                at(&v->c_pixel[k], (size_t)c);
+                at(&v->c_rng[k], (size_t)c);
+                at(&v->c_thr[k], (size_t)c);
+                at(&v->c_w[k], (size_t)c);
+            }
+            at(&v->c_hits, (size_t)c);
+            at(&v->c_merge, (size_t)kMergeRec * c);
+        }), "cudaMalloc");
         v->c_cap = good ? c : 0;
     }
     good = good && ensure_shadow(v, chunk * per);

@@ -39,6 +39,7 @@ using namespace imbart::pt;
 struct imbart_pt_context {
     int device = 0;
     long long cap = 0;       // paths per queue
+    void* block = nullptr;   // the arrays up to scontrib and the grouping's
     float4* rays[2] = {nullptr, nullptr};
     int4* hits = nullptr;
     int* pixel[2] = {nullptr, nullptr};
@@ -63,11 +64,13 @@ struct imbart_pt_context {
     std::vector<unsigned char> graph_key;    // the launch parameters the graph was built with
     int graph_kernels = 0;                   // kernel launches per replay
     int graph_bounces = 0;                   // range state sized for this many bounces
+    void* range_block = nullptr;             // range_state, graph_work and camera
     long long* range_state = nullptr;        // next sample, per-slot totals, waves; then the range's counts
     int* graph_work = nullptr;               // (next, done) counters of the graph's traversal launches
     CameraParams* camera = nullptr;          // the frame's camera and seeding, copied in before the replays
     // Forked form: a second shadow queue, so that a bounce's shadow rays are traced beside the
     // next bounce's closest hits.
+    void* fork_block = nullptr;
     float4* srays2 = nullptr;
     int4* shits2 = nullptr;
     int* spixel2 = nullptr;
@@ -84,25 +87,11 @@ bool ok(cudaError_t e, const char* what) {
     return false;
 }
 
-template <typename T>
-bool dev_alloc(T** p, size_t n, std::vector<void*>* track = nullptr) {
-    *p = nullptr;
-    if (!ok(cudaMalloc((void**)p, sizeof(T) * std::max<size_t>(n, 1)), "cudaMalloc")) return false;
-    if (track) track->push_back(*p);
-    return true;
-}
-
 void free_ctx_buffers(imbart_pt_context* c) {
-    for (int k = 0; k < 2; ++k) {
-        cudaFree(c->rays[k]); cudaFree(c->pixel[k]); cudaFree(c->rng[k]); cudaFree(c->thr[k]); cudaFree(c->bounces[k]);
-        c->rays[k] = nullptr; c->pixel[k] = nullptr; c->rng[k] = nullptr; c->thr[k] = nullptr; c->bounces[k] = nullptr;
-    }
-    cudaFree(c->hits); cudaFree(c->srays); cudaFree(c->shits); cudaFree(c->spixel); cudaFree(c->scontrib);
-    c->hits = nullptr; c->srays = nullptr; c->shits = nullptr; c->spixel = nullptr; c->scontrib = nullptr;
-    cudaFree(c->keys); cudaFree(c->perm); cudaFree(c->tile_counts);
-    c->keys = nullptr; c->perm = nullptr; c->tile_counts = nullptr;
-    cudaFree(c->srays2); cudaFree(c->shits2); cudaFree(c->spixel2); cudaFree(c->scontrib2);
-    c->srays2 = nullptr; c->shits2 = nullptr; c->spixel2 = nullptr; c->scontrib2 = nullptr;
+    cudaFree(c->block);
+    cudaFree(c->fork_block);
+    c->block = c->fork_block = nullptr;
+    c->srays2 = nullptr;
     c->cap = 0;
 }
 
@@ -119,14 +108,24 @@ bool sort_by_material() {
 bool ensure_capacity(imbart_pt_context* c, long long n) {
     if (c->cap >= n) return true;
     free_ctx_buffers(c);
-    bool good = true;
-    for (int k = 0; k < 2 && good; ++k)
-        good = dev_alloc(&c->rays[k], 2 * n) && dev_alloc(&c->pixel[k], n) && dev_alloc(&c->rng[k], n) &&
-               dev_alloc(&c->thr[k], n) && dev_alloc(&c->bounces[k], n);
-    good = good && dev_alloc(&c->hits, n) && dev_alloc(&c->srays, 2 * n) && dev_alloc(&c->shits, n) &&
-           dev_alloc(&c->spixel, n) && dev_alloc(&c->scontrib, n) && dev_alloc(&c->keys, n) &&
-           dev_alloc(&c->perm, n) && dev_alloc(&c->tile_counts, (size_t)kShadeKeys * group_tiles(n));
-    if (!good) { free_ctx_buffers(c); return false; }
+    const bool good = ok(realloc_block(&c->block, [&](BlockLayout& at) {
+        for (int k = 0; k < 2; ++k) {
+            at(&c->rays[k], 2 * (size_t)n);
+            at(&c->pixel[k], (size_t)n);
+            at(&c->rng[k], (size_t)n);
+            at(&c->thr[k], (size_t)n);
+            at(&c->bounces[k], (size_t)n);
+        }
+        at(&c->hits, (size_t)n);
+        at(&c->srays, 2 * (size_t)n);
+        at(&c->shits, (size_t)n);
+        at(&c->spixel, (size_t)n);
+        at(&c->scontrib, (size_t)n);
+        at(&c->keys, (size_t)n);
+        at(&c->perm, (size_t)n);
+        at(&c->tile_counts, (size_t)kShadeKeys * group_tiles(n));
+    }), "cudaMalloc");
+    if (!good) return false;
     c->cap = n;
     c->graph_key.clear();   // the frame graph names the old buffers
     return true;
@@ -207,18 +206,16 @@ std::vector<unsigned char> frame_key(const imbart_scene* scene, const imbart_sha
 }
 
 bool ensure_range_state(imbart_pt_context* c, int bounces, cudaStream_t st) {
-    if (!c->camera && !ok(cudaMalloc((void**)&c->camera, sizeof(CameraParams)), "cudaMalloc")) return false;
     if (c->graph_bounces >= bounces) return true;
-    cudaFree(c->range_state);
-    cudaFree(c->graph_work);
-    c->range_state = nullptr;
-    c->graph_work = nullptr;
     c->graph_bounces = 0;
     c->graph_key.clear();
     const int n_slots = 2 * bounces + 2;
     const size_t state_bytes = sizeof(long long) * (n_slots + 2) + sizeof(int) * n_slots;
-    if (!ok(cudaMalloc((void**)&c->range_state, state_bytes), "cudaMalloc") ||
-        !ok(cudaMalloc((void**)&c->graph_work, sizeof(int) * 4 * bounces), "cudaMalloc") ||
+    if (!ok(realloc_block(&c->range_block, [&](BlockLayout& at) {
+            at(&c->range_state, (state_bytes + sizeof(long long) - 1) / sizeof(long long));
+            at(&c->graph_work, 4 * (size_t)bounces);
+            at(&c->camera, 1);
+        }), "cudaMalloc") ||
         !ok(cudaMemsetAsync(c->graph_work, 0, sizeof(int) * 4 * bounces, st), "cudaMemsetAsync"))
         return false;
     c->graph_bounces = bounces;
@@ -293,9 +290,13 @@ int build_range_graph(imbart_pt_context* ctx, const imbart_scene* scene, const i
     const int n_slots = 2 * max_path_len + 2;
     long long* state = ctx->range_state;
     int* counts = reinterpret_cast<int*>(state + n_slots + 2);
-    if (fork && !ctx->srays2 &&
-        !(dev_alloc(&ctx->srays2, 2 * chunk) && dev_alloc(&ctx->shits2, chunk) && dev_alloc(&ctx->spixel2, chunk) &&
-          dev_alloc(&ctx->scontrib2, chunk)))
+    // As large as the first queue: a later frame's range may be larger than this one's.
+    if (fork && !ctx->srays2 && !ok(realloc_block(&ctx->fork_block, [&](BlockLayout& at) {
+            at(&ctx->srays2, 2 * (size_t)ctx->cap);
+            at(&ctx->shits2, (size_t)ctx->cap);
+            at(&ctx->spixel2, (size_t)ctx->cap);
+            at(&ctx->scontrib2, (size_t)ctx->cap);
+        }), "cudaMalloc"))
         return IMBART_ERR_OUT_OF_MEMORY;
     GraphBuilder gb;
     if (!ok(cudaGraphCreate(&gb.graph, 0), "cudaGraphCreate")) return IMBART_ERR_CUDA;
@@ -561,9 +562,7 @@ void imbart_pt_destroy(imbart_pt_context* c) {
     cudaFree(c->work);
     if (c->ev[0]) { cudaEventDestroy(c->ev[0]); cudaEventDestroy(c->ev[1]); }
     if (c->exec) cudaGraphExecDestroy(c->exec);
-    cudaFree(c->range_state);
-    cudaFree(c->graph_work);
-    cudaFree(c->camera);
+    cudaFree(c->range_block);
     cudaSetDevice(prev);
     delete c;
 }
