@@ -248,8 +248,9 @@ int64_t imbart_kernel_launch_count(void);
  * many lanes are idle; postpone_lanes (0..32): triangle tests are postponed while fewer than
  * postpone_lanes/32 of the live lanes would test together (0 = never).
  * imbart_set_trace_config sets the variant of both query types; imbart_set_trace_variant_any
- * then overrides the any-hit one. Defaults: closest 4, any-hit 6, refill 24, postpone 0
- * (environment: IMBART_TRACE_VARIANT, _VARIANT_ANY, _REFILL, _POSTPONE). */
+ * then overrides the any-hit one. Defaults: incoherent closest hits 17 with refill 8, any hits 11
+ * with 8, coherent closest hits 11 with 24, postpone 0 (environment: IMBART_TRACE_VARIANT,
+ * _VARIANT_ANY, _REFILL, _POSTPONE). */
 int imbart_set_trace_config(int variant, int refill_lanes, int postpone_lanes);
 int imbart_set_trace_variant_any(int variant);
 int imbart_get_trace_config(int* variant, int* refill_lanes, int* postpone_lanes);
