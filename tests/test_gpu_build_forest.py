@@ -80,3 +80,40 @@ def test_forest_build_and_refit(cuda, name):
         got, _ = trace(ds, rays)
         assert H.hits_equal(want, got).all()
     ds.close()
+
+
+@pytest.mark.gpu
+def test_scratch_between_builds(cuda):
+    """The scratch kept from one build to the next: smaller and larger scenes after each other, given
+    back between builds, and two threads building at once; every build's arrays are the first one's."""
+    import threading
+    from imbatracer_b200 import native as N
+    scenes = [forest(n) for n in ("tiny trees", "one", "large", "edges")]
+
+    def arrays(k):
+        ds = S.DeviceScene.build_gpu(*scenes[k])
+        out = [records(ds, 0, int(ds.info.wide_nodes), 80), records(ds, 1, int(ds.info.triangles), 48)]
+        ds.close()
+        return out
+
+    def same(k):
+        return all(np.array_equal(a, b) for a, b in zip(first[k], arrays(k)))
+
+    first = [arrays(k) for k in range(4)]
+    for k in (1, 2, 0, 3, 2):
+        assert same(k), k
+        if k == 2:
+            N.load().imbart_invalidate_scenes()
+    wrong = []
+
+    def work(order):
+        try:
+            wrong.extend(k for k in order if not same(k))
+        except Exception as e:          # shown by the assertion below
+            wrong.append(repr(e))
+    threads = [threading.Thread(target=work, args=(o,)) for o in ([0, 1, 2, 3] * 2, [2, 3, 0, 1] * 2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert wrong == []
