@@ -130,9 +130,11 @@ void trace_config_snapshot(int out[10]);
 // leaving the rest of the SMs to concurrent work on other streams.
 void scene_set_grid_share(imbart_scene* s, float share);
 
-// Every scene value a traversal launch takes into its parameters (array pointers, root,
-// masks, device): two launches with equal keys and arguments are the same launch.
-void scene_launch_key(const imbart_scene* s, unsigned long long out[12]);
+// Every scene value a traversal launch takes into its parameters or chooses its kernel by (array
+// pointers, root, direct root and instance, node width, masks, device): two launches with equal
+// keys and arguments are the same launch.
+constexpr int kSceneKeyWords = 14;
+void scene_launch_key(const imbart_scene* s, unsigned long long out[kSceneKeyWords]);
 
 // Device arrays of a built photon grid (hashgrid.cu): photons in bucket order (float4 xyz +
 // index bits), inclusive bucket ends, the 10 grid parameters; false before the first build.

@@ -499,7 +499,7 @@ void scene_set_grid_share(imbart_scene* s, float share) {
     s->grid_share = !(share > 0.05f) ? 0.05f : (share < 1.0f ? share : 1.0f);
 }
 
-void scene_launch_key(const imbart_scene* s, unsigned long long out[12]) {
+void scene_launch_key(const imbart_scene* s, unsigned long long out[kSceneKeyWords]) {
     out[0] = (unsigned long long)(uintptr_t)s->nodes; out[1] = (unsigned long long)(uintptr_t)s->tris;
     out[2] = (unsigned long long)(uintptr_t)s->insts; out[3] = (unsigned long long)(uintptr_t)s->indices;
     out[4] = (unsigned long long)(uintptr_t)s->texcoords; out[5] = (unsigned long long)(uintptr_t)s->masks;
@@ -509,6 +509,8 @@ void scene_launch_key(const imbart_scene* s, unsigned long long out[12]) {
     std::memcpy(&share_bits, &s->grid_share, sizeof(share_bits));
     out[10] = (unsigned long long)s->info.masked | ((unsigned long long)share_bits << 32);
     out[11] = (unsigned long long)s->device;
+    out[12] = (unsigned long long)(unsigned)s->direct_root | ((unsigned long long)(unsigned)s->direct_inst << 32);
+    out[13] = (unsigned long long)(unsigned)s->info.node_width;
 }
 
 void trace_config_snapshot(int out[10]) {

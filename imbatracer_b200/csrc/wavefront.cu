@@ -180,7 +180,7 @@ __global__ void range_end_kernel(long long* state, const int* counts, int n_slot
 // Everything the graph's kernels take into their parameters: equal keys, same graph. The
 // camera and the seed are read on the device, so a new view or seed replays the same graph.
 struct FrameGraphKey {
-    unsigned long long scene[12];
+    unsigned long long scene[kSceneKeyWords];
     ShadingScene s;
     float* image;
     long long total, chunk;
