@@ -111,9 +111,9 @@ __global__ void __launch_bounds__(kBlock) bounds_kernel(const float* __restrict_
     for (int i = first; i < n; i += step) {
         const float* p = pos + (size_t)i * stride;
         for (int a = 0; a < 3; ++a) {
-            const float v = p[a];
-            lo[a] = lo[a] < v ? lo[a] : v;
-            hi[a] = hi[a] > v ? hi[a] : v;
+            const float v = p[a];    // a NaN is no position: it is kept out of both
+            lo[a] = v < lo[a] ? v : lo[a];
+            hi[a] = v > hi[a] ? v : hi[a];
         }
     }
     __syncthreads();
