@@ -347,10 +347,9 @@ imbart_hashgrid* imbart_hashgrid_create(int device) {
     cudaGetDevice(&prev);
     cudaSetDevice(device);
     // The parameters, then the builds' state words, zero until the first build.
-    const bool good = ok(cudaMalloc((void**)&g->params, sizeof(float) * 16 + sizeof(unsigned) * kStateWords),
-                         "cudaMalloc") &&
-                      ok(cudaMemset(g->params, 0, sizeof(float) * 16 + sizeof(unsigned) * kStateWords), "cudaMemset") &&
-                      ok(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
+    const size_t bytes = sizeof(float) * 16 + sizeof(unsigned) * kStateWords;
+    const bool good = ok(cudaMalloc((void**)&g->params, bytes), "cudaMalloc") &&
+                      ok(zero_now(g->params, bytes), "cudaMemsetAsync");
     cudaSetDevice(prev);
     if (!good) { cudaFree(g->params); delete g; return nullptr; }
     g->state = reinterpret_cast<unsigned*>(g->params + 16);

@@ -1107,8 +1107,8 @@ imbart_vcm* imbart_vcm_create(int device) {
                       ok(cudaEventCreateWithFlags(&v->queue[0].done, cudaEventDisableTiming), "cudaEventCreate") &&
                       ok(cudaEventCreateWithFlags(&v->queue[1].done, cudaEventDisableTiming), "cudaEventCreate") &&
                       ok(cudaMalloc((void**)&v->counts, sizeof(int) * 9), "cudaMalloc") &&
-                      ok(cudaMemset(v->counts, 0, sizeof(int) * 9), "cudaMemset") &&
-                      ok(cudaDeviceSynchronize(), "cudaDeviceSynchronize") &&
+                      ok(cudaMemsetAsync(v->counts, 0, sizeof(int) * 9, v->side), "cudaMemsetAsync") &&
+                      ok(cudaStreamSynchronize(v->side), "cudaStreamSynchronize") &&
                       ok(cudaMallocHost((void**)&v->host_counts, sizeof(int) * 4), "cudaMallocHost") &&
                       (v->grid = imbart_hashgrid_create(device)) != nullptr;
     cudaSetDevice(prev);
