@@ -910,12 +910,12 @@ int trace_shadows(imbart_vcm* v, const imbart_scene* scene, const VcmParams& p, 
     if (!ok(cudaEventRecord(v->shaded, s), "cudaEventRecord") ||
         !ok(cudaStreamWaitEvent(v->side, v->shaded, 0), "cudaStreamWaitEvent"))
         return IMBART_ERR_CUDA;
+    q.used = true;    // from the first launch on: a pass that fails here still waits for the side stream
     const int rc = launch_trace_internal(scene, q.rays, q.hits, nullptr, bound, IMBART_TRACE_ANY, v->side, nullptr,
                                          nullptr, p.counts + 1);
     if (rc) return rc;
     vcm_shadow_kernel<<<(bound + 127) / 128, 128, 0, v->side>>>(p.counts + 1, q.hits, q.pixel, q.contrib, p.image);
     note_launches(1);
-    q.used = true;
     return ok(cudaGetLastError(), "shadow kernel") && ok(cudaEventRecord(q.done, v->side), "cudaEventRecord")
                ? 0
                : IMBART_ERR_CUDA;
