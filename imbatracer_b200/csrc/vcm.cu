@@ -872,6 +872,11 @@ bool valid_settings(const imbart_vcm_settings* st) {
            st->grid_table_size >= 0;
 }
 
+// What an algorithm's passes fill: photon mapping queues no shadow rays, light tracing stores no
+// light vertices (light_shade_kernel, vcm_camera_shade_kernel), so they hold no room for them.
+bool casts_shadows(const imbart_vcm_settings* st) { return st->algorithm != IMBART_PPM; }
+bool stores_vertices(const imbart_vcm_settings* st) { return st->algorithm != IMBART_LT; }
+
 bool ensure_shadow(imbart_vcm* v, long long need) {
     if (v->s_cap >= need) return true;
     need = std::max(need, v->s_cap * 3 / 2);   // geometric growth: reallocation synchronizes the device
@@ -910,6 +915,7 @@ int trace_shadows(imbart_vcm* v, const imbart_scene* scene, const VcmParams& p, 
     if (!ok(cudaEventRecord(v->shaded, s), "cudaEventRecord") ||
         !ok(cudaStreamWaitEvent(v->side, v->shaded, 0), "cudaStreamWaitEvent"))
         return IMBART_ERR_CUDA;
+    if (p.algo == kAlgoPpm) return 0;    // no shadow rays
     q.used = true;    // from the first launch on: a pass that fails here still waits for the side stream
     const int rc = launch_trace_internal(scene, q.rays, q.hits, nullptr, bound, IMBART_TRACE_ANY, v->side, nullptr,
                                          nullptr, p.counts + 1);
@@ -1207,7 +1213,7 @@ int imbart_vcm_light_pass_range(imbart_vcm* v, const imbart_scene* scene, const 
         good = ok(cudaMalloc((void**)&v->d_tiles, tiles.size() * sizeof(LightTile)), "cudaMalloc");
         v->tiles_cap = good ? (long long)tiles.size() : 0;
     }
-    good = good && ensure_shadow(v, P);
+    good = good && (!casts_shadows(st) || ensure_shadow(v, P));
     if (!good) { cudaSetDevice(prev); return IMBART_ERR_OUT_OF_MEMORY; }
     if (!ok(cudaMemcpyAsync(v->d_tiles, tiles.data(), sizeof(LightTile) * tiles.size(), cudaMemcpyHostToDevice, s),
             "cudaMemcpyAsync")) {
@@ -1221,6 +1227,7 @@ int imbart_vcm_light_pass_range(imbart_vcm* v, const imbart_scene* scene, const 
     note_launches(1);
     int rc = 0;
     long long n_closest = 0, n_shadow = 0, n_waves = 0;
+    const bool stores = stores_vertices(st);
     int live = P;
     int n = P;   // slots in use: the live paths after the last compaction, in path order
     while (live > 0 && !rc) {
@@ -1247,20 +1254,22 @@ int imbart_vcm_light_pass_range(imbart_vcm* v, const imbart_scene* scene, const 
         if (rc) break;
         n_closest += live;
         ++n_waves;
-        // Room for up to n new vertices before the wavefront appends (a larger cache takes over the
-        // vertices once the last append on s is done). A new context starts with two per path: light
-        // passes leave 1.5 to 2.
-        long long room = 7ll * (v->cache_count + (long long)n);
-        if (v->cache_cap == 0) room *= 2;
-        if (v->cache_cap < room && !ok(cudaStreamSynchronize(s), "cudaStreamSynchronize")) {
-            rc = IMBART_ERR_CUDA;
-            break;
+        if (stores) {
+            // Room for up to n new vertices before the wavefront appends (a larger cache takes over
+            // the vertices once the last append on s is done). A new context starts with two per
+            // path: light passes leave 1.5 to 2.
+            long long room = 7ll * (v->cache_count + (long long)n);
+            if (v->cache_cap == 0) room *= 2;
+            if (v->cache_cap < room && !ok(cudaStreamSynchronize(s), "cudaStreamSynchronize")) {
+                rc = IMBART_ERR_CUDA;
+                break;
+            }
+            if (!grow(&v->cache, &v->cache_cap, room, 7ll * v->cache_count)) {
+                rc = IMBART_ERR_OUT_OF_MEMORY;
+                break;
+            }
+            p.cache = v->cache;
         }
-        if (!grow(&v->cache, &v->cache_cap, room, 7ll * v->cache_count)) {
-            rc = IMBART_ERR_OUT_OF_MEMORY;
-            break;
-        }
-        p.cache = v->cache;
         if (!group_paths(v, sh, n, s, LightKeys{p.s, v->l_hits, v->l_thr})) {
             rc = IMBART_ERR_CUDA;
             break;
@@ -1268,20 +1277,27 @@ int imbart_vcm_light_pass_range(imbart_vcm* v, const imbart_scene* scene, const 
         light_shade_kernel<<<grid_n, 128, 0, s>>>(p, n, v->l_rays, v->l_hits, v->l_rng, v->l_thr, v->l_w, v->stage,
                                                   v->vflags, q->rays, q->pixel, q->contrib,
                                                   v->use_perm ? v->perm : nullptr);
-        slot_scan_kernel<<<n_blocks_n, kScanBlock, 0, s>>>(v->vflags, nullptr, n, v->bsums,
-                                                           reinterpret_cast<unsigned*>(v->counts + 8));
+        note_launches(1);
+        v->host_counts[3] = 0;
+        if (stores) {
+            slot_scan_kernel<<<n_blocks_n, kScanBlock, 0, s>>>(v->vflags, nullptr, n, v->bsums,
+                                                               reinterpret_cast<unsigned*>(v->counts + 8));
+            note_launches(1);
+        }
         if (!ok(cudaMemcpyAsync(v->host_counts, p.counts, sizeof(int) * 3, cudaMemcpyDeviceToHost, s),
                 "cudaMemcpyAsync") ||
-            !ok(cudaMemcpyAsync(v->host_counts + 3, v->bsums + n_blocks_n, sizeof(int), cudaMemcpyDeviceToHost, s),
-                "cudaMemcpyAsync")) {
+            (stores && !ok(cudaMemcpyAsync(v->host_counts + 3, v->bsums + n_blocks_n, sizeof(int),
+                                           cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync"))) {
             rc = IMBART_ERR_CUDA;
             break;
         }
         rc = trace_shadows(v, scene, p, *q, n, s);
         if (rc) break;
-        vertex_scatter_kernel<<<n_blocks_n, kScanBlock, 0, s>>>(v->vflags, n, v->bsums, v->stage, v->cache,
-                                                                v->cache_count);
-        note_launches(3);
+        if (stores) {
+            vertex_scatter_kernel<<<n_blocks_n, kScanBlock, 0, s>>>(v->vflags, n, v->bsums, v->stage, v->cache,
+                                                                    v->cache_count);
+            note_launches(1);
+        }
         if (!ok(cudaGetLastError(), "light pass kernels") ||
             !ok(cudaEventSynchronize(v->shaded), "cudaEventSynchronize")) {
             rc = IMBART_ERR_CUDA;
@@ -1394,7 +1410,7 @@ int imbart_vcm_camera_pass_range(imbart_vcm* v, const imbart_scene* scene, const
         }), "cudaMalloc");
         v->c_cap = good ? c : 0;
     }
-    good = good && ensure_shadow(v, chunk * per);
+    good = good && (!casts_shadows(st) || ensure_shadow(v, chunk * per));
     if (!good) { cudaSetDevice(prev); return IMBART_ERR_OUT_OF_MEMORY; }
     VcmParams p = make_params(v, sh, cam, st, image);
     long long n_closest = 0, n_shadow = 0, n_waves = 0;
