@@ -838,7 +838,8 @@ struct imbart_vcm {
     // Two shadow queues: a wavefront's shadow rays are traced and accumulated on a stream of
     // their own beside the next wavefront (begin_wave / trace_shadows).
     void* s_block = nullptr;
-    long long s_cap = 0;
+    long long s_cap = 0;            // rays per queue
+    int s_queues = 2;               // queues held: one where a second finds no room
     imbart::ShadowQueue queue[2];
     cudaStream_t side = nullptr;
     cudaEvent_t shaded = nullptr;
@@ -877,19 +878,49 @@ bool valid_settings(const imbart_vcm_settings* st) {
 bool casts_shadows(const imbart_vcm_settings* st) { return st->algorithm != IMBART_PPM; }
 bool stores_vertices(const imbart_vcm_settings* st) { return st->algorithm != IMBART_LT; }
 
-bool ensure_shadow(imbart_vcm* v, long long need) {
-    if (v->s_cap >= need) return true;
-    need = std::max(need, v->s_cap * 3 / 2);   // geometric growth: reallocation synchronizes the device
-    const size_t c = (size_t)need;
-    const bool good = ok(realloc_block(&v->s_block, [&](BlockLayout& at) {
-        for (ShadowQueue& q : v->queue) {
+// Shadow queues of `cap` rays each.
+cudaError_t alloc_queues(imbart_vcm* v, int queues, long long cap) {
+    const size_t c = (size_t)cap;
+    const cudaError_t e = realloc_block(&v->s_block, [&](BlockLayout& at) {
+        for (int k = 0; k < queues; ++k) {
+            ShadowQueue& q = v->queue[k];
             at(&q.rays, 2 * c);
             at(&q.hits, c);
             at(&q.pixel, c);
             at(&q.contrib, c);
         }
-    }), "cudaMalloc");
-    v->s_cap = good ? need : 0;
+    });
+    v->s_cap = e == cudaSuccess ? cap : 0;
+    v->s_queues = queues;
+    return e;
+}
+
+bool ensure_shadow(imbart_vcm* v, long long need) {
+    if (v->s_cap >= need) return true;
+    need = std::max(need, v->s_cap * 3 / 2);   // geometric growth: reallocation synchronizes the device
+    // The second queue only makes passes faster: where it finds no room they go on with one.
+    if (alloc_queues(v, 2, need) == cudaSuccess) return true;
+    (void)cudaGetLastError();
+    return ok(alloc_queues(v, 1, need), "cudaMalloc");
+}
+
+// Runs `alloc` (true on success; it records its own error). Where it finds no memory, the second
+// shadow queue is given back and it is run again: no wavefront stands in a queue then but those
+// whose rays the side stream still traces.
+template <typename Alloc>
+bool with_room(imbart_vcm* v, cudaStream_t s, const Alloc& alloc) {
+    const int code = imbart_last_error();
+    const std::string msg = imbart_last_error_string();
+    bool good = alloc();
+    if (!good && imbart_last_error() == IMBART_ERR_OUT_OF_MEMORY && v->s_cap > 0 && v->s_queues == 2) {
+        (void)cudaGetLastError();
+        if (!ok(cudaStreamSynchronize(s), "cudaStreamSynchronize") ||
+            !ok(cudaStreamSynchronize(v->side), "cudaStreamSynchronize") ||
+            !ok(alloc_queues(v, 1, v->s_cap), "cudaMalloc"))
+            return false;
+        good = alloc();
+    }
+    if (good) set_error(code, msg);   // what an attempt recorded on the way
     return good;
 }
 
@@ -901,8 +932,9 @@ bool ensure_shadow(imbart_vcm* v, long long need) {
 
 // Wavefront `wave` of a pass: its shadow queue, free again on stream s, with zeroed counts.
 bool begin_wave(imbart_vcm* v, long long wave, cudaStream_t s, VcmParams& p, ShadowQueue*& q) {
-    q = &v->queue[wave & 1];
-    p.counts = v->counts + 4 * (wave & 1);
+    const int k = v->s_queues == 2 ? (int)(wave & 1) : 0;
+    q = &v->queue[k];
+    p.counts = v->counts + 4 * k;
     return (!q->used || ok(cudaStreamWaitEvent(s, q->done, 0), "cudaStreamWaitEvent")) &&
            ok(cudaMemsetAsync(p.counts, 0, sizeof(int) * 4, s), "cudaMemsetAsync");
 }
@@ -944,11 +976,13 @@ bool group_paths(imbart_vcm* v, const imbart_shading* sh, int n, cudaStream_t s,
     if (!v->use_perm) return true;
     if (v->sort_cap < n) {
         const long long c = std::max<long long>(n, v->sort_cap * 3 / 2);
-        const bool good = ok(realloc_block(&v->sort_block, [&](BlockLayout& at) {
-            at(&v->keys, (size_t)c);
-            at(&v->perm, (size_t)c);
-            at(&v->tile_counts, (size_t)pt::kShadeKeys * pt::group_tiles(c));
-        }), "cudaMalloc");
+        const bool good = with_room(v, s, [&] {
+            return ok(realloc_block(&v->sort_block, [&](BlockLayout& at) {
+                at(&v->keys, (size_t)c);
+                at(&v->perm, (size_t)c);
+                at(&v->tile_counts, (size_t)pt::kShadeKeys * pt::group_tiles(c));
+            }), "cudaMalloc");
+        });
         v->sort_cap = good ? c : 0;
         if (!good) return false;
     }
@@ -1028,6 +1062,12 @@ int build_grid(imbart_vcm* v, const imbart_vcm_settings* st, cudaStream_t s) {
     const int rc = imbart_hashgrid_build(v->grid, reinterpret_cast<const float*>(v->cache), 28, v->cache_count,
                                          v->pm_radius, cell_factor, st->grid_table_size, s);
     v->grid_built = rc == 0;
+    return rc;
+}
+
+int grid_with_room(imbart_vcm* v, const imbart_vcm_settings* st, cudaStream_t s) {
+    int rc = 0;
+    with_room(v, s, [&] { return (rc = build_grid(v, st, s)) == 0; });
     return rc;
 }
 
@@ -1191,20 +1231,22 @@ int imbart_vcm_light_pass_range(imbart_vcm* v, const imbart_scene* scene, const 
     if (v->l_cap < P) {
         const long long c = std::max<long long>(P, v->l_cap * 3 / 2);
         const long long cb = (c + kScanTile - 1) / kScanTile;
-        good = ok(realloc_block(&v->l_block, [&](BlockLayout& at) {
-            at(&v->l_rays, 2 * (size_t)c);
-            at(&v->l_hits, (size_t)c);
-            at(&v->l_rng, (size_t)c);
-            at(&v->l_thr, (size_t)c);
-            at(&v->l_w, (size_t)c);
-            at(&v->l_rays2, 2 * (size_t)c);
-            at(&v->l_rng2, (size_t)c);
-            at(&v->l_thr2, (size_t)c);
-            at(&v->l_w2, (size_t)c);
-            at(&v->stage, 7 * (size_t)c);
-            at(&v->vflags, (size_t)c);
-            at(&v->bsums, (size_t)cb + 1);
-        }), "cudaMalloc");
+        good = with_room(v, s, [&] {
+            return ok(realloc_block(&v->l_block, [&](BlockLayout& at) {
+                at(&v->l_rays, 2 * (size_t)c);
+                at(&v->l_hits, (size_t)c);
+                at(&v->l_rng, (size_t)c);
+                at(&v->l_thr, (size_t)c);
+                at(&v->l_w, (size_t)c);
+                at(&v->l_rays2, 2 * (size_t)c);
+                at(&v->l_rng2, (size_t)c);
+                at(&v->l_thr2, (size_t)c);
+                at(&v->l_w2, (size_t)c);
+                at(&v->stage, 7 * (size_t)c);
+                at(&v->vflags, (size_t)c);
+                at(&v->bsums, (size_t)cb + 1);
+            }), "cudaMalloc");
+        });
         v->l_cap = good ? c : 0;
     }
     if (good && v->tiles_cap < (long long)tiles.size()) {
@@ -1248,32 +1290,34 @@ int imbart_vcm_light_pass_range(imbart_vcm* v, const imbart_scene* scene, const 
         }
         const int grid_n = (n + 127) / 128;
         const int n_blocks_n = (n + kScanTile - 1) / kScanTile;
-        ShadowQueue* q = nullptr;
-        if (!begin_wave(v, n_waves, s, p, q)) { rc = IMBART_ERR_CUDA; break; }
         rc = launch_trace_internal(scene, v->l_rays, v->l_hits, nullptr, n, IMBART_TRACE_CLOSEST, s, nullptr);
         if (rc) break;
         n_closest += live;
-        ++n_waves;
         if (stores) {
             // Room for up to n new vertices before the wavefront appends (a larger cache takes over
             // the vertices once the last append on s is done). A new context starts with two per
             // path: light passes leave 1.5 to 2.
-            long long room = 7ll * (v->cache_count + (long long)n);
-            if (v->cache_cap == 0) room *= 2;
+            const long long room = 7ll * (v->cache_count + (long long)n);
             if (v->cache_cap < room && !ok(cudaStreamSynchronize(s), "cudaStreamSynchronize")) {
                 rc = IMBART_ERR_CUDA;
                 break;
             }
-            if (!grow(&v->cache, &v->cache_cap, room, 7ll * v->cache_count)) {
+            if (!with_room(v, s, [&] {
+                    if (v->cache_cap == 0 && grow(&v->cache, &v->cache_cap, 2 * room)) return true;
+                    (void)cudaGetLastError();
+                    return grow(&v->cache, &v->cache_cap, room, 7ll * v->cache_count);
+                })) {
                 rc = IMBART_ERR_OUT_OF_MEMORY;
                 break;
             }
             p.cache = v->cache;
         }
-        if (!group_paths(v, sh, n, s, LightKeys{p.s, v->l_hits, v->l_thr})) {
+        ShadowQueue* q = nullptr;
+        if (!group_paths(v, sh, n, s, LightKeys{p.s, v->l_hits, v->l_thr}) || !begin_wave(v, n_waves, s, p, q)) {
             rc = IMBART_ERR_CUDA;
             break;
         }
+        ++n_waves;
         light_shade_kernel<<<grid_n, 128, 0, s>>>(p, n, v->l_rays, v->l_hits, v->l_rng, v->l_thr, v->l_w, v->stage,
                                                   v->vflags, q->rays, q->pixel, q->contrib,
                                                   v->use_perm ? v->perm : nullptr);
@@ -1308,7 +1352,7 @@ int imbart_vcm_light_pass_range(imbart_vcm* v, const imbart_scene* scene, const 
         if (n_waves <= wave_cap) wave_counts[n_waves - 1] = v->host_counts[3];
         live = v->host_counts[2];
     }
-    if (!rc) rc = build_grid(v, st, s);
+    if (!rc) rc = grid_with_room(v, st, s);
     rc = end_pass(v, rc, s);
     if (stats) { stats[0] = n_closest; stats[1] = n_shadow; stats[2] = n_waves; }
     cudaSetDevice(prev);
@@ -1354,13 +1398,14 @@ int imbart_vcm_load_light_vertices(imbart_vcm* v, const imbart_vcm_settings* st,
     cudaGetDevice(&prev);
     cudaSetDevice(v->device);
     int rc = 0;
-    if (!grow(&v->cache, &v->cache_cap, 7ll * std::max(count, 1))) rc = IMBART_ERR_OUT_OF_MEMORY;
+    if (!with_room(v, s, [&] { return grow(&v->cache, &v->cache_cap, 7ll * std::max(count, 1)); }))
+        rc = IMBART_ERR_OUT_OF_MEMORY;
     if (!rc && count > 0 &&
         !ok(cudaMemcpyAsync(v->cache, vertices, sizeof(float) * 28 * (size_t)count, cudaMemcpyDefault, s),
             "cudaMemcpyAsync"))
         rc = IMBART_ERR_CUDA;
     v->cache_count = rc ? 0 : count;
-    if (!rc) rc = build_grid(v, st, s);
+    if (!rc) rc = grid_with_room(v, st, s);
     cudaSetDevice(prev);
     return rc;
 }
@@ -1397,17 +1442,19 @@ int imbart_vcm_camera_pass_range(imbart_vcm* v, const imbart_scene* scene, const
     bool good = true;
     if (v->c_cap < chunk) {
         const long long c = std::max(chunk, v->c_cap * 3 / 2);
-        good = ok(realloc_block(&v->c_block, [&](BlockLayout& at) {
-            for (int k = 0; k < 2; ++k) {
-                at(&v->c_rays[k], 2 * (size_t)c);
-                at(&v->c_pixel[k], (size_t)c);
-                at(&v->c_rng[k], (size_t)c);
-                at(&v->c_thr[k], (size_t)c);
-                at(&v->c_w[k], (size_t)c);
-            }
-            at(&v->c_hits, (size_t)c);
-            at(&v->c_merge, (size_t)kMergeRec * c);
-        }), "cudaMalloc");
+        good = with_room(v, s, [&] {
+            return ok(realloc_block(&v->c_block, [&](BlockLayout& at) {
+                for (int k = 0; k < 2; ++k) {
+                    at(&v->c_rays[k], 2 * (size_t)c);
+                    at(&v->c_pixel[k], (size_t)c);
+                    at(&v->c_rng[k], (size_t)c);
+                    at(&v->c_thr[k], (size_t)c);
+                    at(&v->c_w[k], (size_t)c);
+                }
+                at(&v->c_hits, (size_t)c);
+                at(&v->c_merge, (size_t)kMergeRec * c);
+            }), "cudaMalloc");
+        });
         v->c_cap = good ? c : 0;
     }
     good = good && (!casts_shadows(st) || ensure_shadow(v, chunk * per));
@@ -1423,17 +1470,16 @@ int imbart_vcm_camera_pass_range(imbart_vcm* v, const imbart_scene* scene, const
                                                          v->c_pixel[cur], v->c_rng[cur], v->c_thr[cur], v->c_w[cur]);
         note_launches(1);
         while (n > 0 && !rc) {
-            ShadowQueue* q = nullptr;
-            if (!begin_wave(v, n_waves, s, p, q)) { rc = IMBART_ERR_CUDA; break; }
             rc = launch_trace_internal(scene, v->c_rays[cur], v->c_hits, nullptr, n, IMBART_TRACE_CLOSEST, s, nullptr);
             if (rc) break;
             n_closest += n;
-            ++n_waves;
             const int nxt = 1 - cur;
-            if (!group_paths(v, sh, n, s, pt::HitKeys{p.s, v->c_hits})) {
+            ShadowQueue* q = nullptr;
+            if (!group_paths(v, sh, n, s, pt::HitKeys{p.s, v->c_hits}) || !begin_wave(v, n_waves, s, p, q)) {
                 rc = IMBART_ERR_CUDA;
                 break;
             }
+            ++n_waves;
             vcm_camera_shade_kernel<<<(n + 127) / 128, 128, 0, s>>>(
                 p, n, v->c_rays[cur], v->c_hits, v->c_pixel[cur], v->c_rng[cur], v->c_thr[cur], v->c_w[cur],
                 v->c_rays[nxt], v->c_pixel[nxt], v->c_rng[nxt], v->c_thr[nxt], v->c_w[nxt], q->rays, q->pixel,

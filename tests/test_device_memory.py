@@ -1,9 +1,39 @@
-"""Device memory that calls take: algorithms hold no buffers they never fill."""
+"""Device memory that calls take: what fits without the second copy of a buffer that only makes a
+call faster still fits, and algorithms hold no buffers they never fill."""
+import gc
+
+import numpy as np
 import pytest
 
+from imbatracer_b200 import native as N
+from imbatracer_b200 import scenegen as G
 from tests.test_pt import small_mixed_scene
 
 MB = 1 << 20
+
+
+class Filled:
+    """All device memory taken but `left` bytes."""
+
+    def __init__(self, left):
+        import torch
+        gc.collect()
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        N.load().imbart_invalidate_scenes()
+        N.load().imbart_clear_error()
+        free = torch.cuda.mem_get_info()[0]
+        self.block = torch.empty(max(free - left, 0), dtype=torch.uint8, device="cuda")
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        import torch
+        del self.block
+        torch.cuda.empty_cache()
+        N.load().imbart_invalidate_scenes()
+        N.load().imbart_clear_error()
 
 
 def held_by(run):
@@ -51,3 +81,71 @@ def test_photon_mapping_holds_no_shadow_rays(cuda):
     run().close()
     # 292 B a camera path, 1,000 light paths and 2,000 vertices; a shadow queue would be 6.9 KB a path.
     assert held_by(run) <= 292 * w * h + 12 * MB
+
+
+@pytest.mark.gpu
+def test_connections_fit_with_one_shadow_queue(cuda):
+    """A camera pass whose shadow rays fit once but not twice."""
+    from imbatracer_b200.integrators import GpuScene, VcmIntegrator
+    gs = GpuScene(small_mixed_scene())
+    w, h, conn = 512, 384, 127
+
+    def image(left=None):
+        vi = VcmIntegrator(gs, "bpt", w, h, max_path_len=3, light_path_count=500, num_connections=conn)
+        vi.begin_iteration(1)
+        vi.light_pass(3)
+        img = vi._image(None)
+        vi._image(None)                                        # memory for the test's own tensors
+        if left is None:
+            vi.camera_pass(4, img)
+        else:
+            with Filled(left):
+                vi.camera_pass(4, img)
+                assert N.last_error()[0] == 0
+        out = img.cpu().numpy().astype(np.float64)
+        vi.close()
+        return out
+    ref = image()
+    queue = 68 * (1 + conn) * w * h                            # 1.7 GB
+    got = image(queue + 512 * MB)
+    # Each pixel sums at most 3 * (conn + 2) float32 terms, in another order.
+    assert (np.abs(got - ref) <= 3 * (conn + 2) * 2.0 ** -24 * np.maximum(ref, 1e-6)).all()
+
+
+def mirrors():
+    """A mirror ball over a mirror ground: light paths that leave no vertices."""
+    rng = np.random.default_rng(2)
+    mirror = G.Material(G.MIRROR, color=(0.9, 0.9, 0.9), eta=0.2, kappa=3.0)
+    parts = [(*G.displaced_sphere(rng, 2, (0, 0, 0), 1.0), 0),
+             (*G.quad([-20, -1.6, -20], [-20, -1.6, 20], [20, -1.6, 20], [20, -1.6, -20]), 0),
+             (np.array([[-3, 6, -2], [3, 6, 2], [3, 6, -2]], np.float32), np.array([[0, 1, 2]], np.int32), 1)]
+    e = (30.0, 28.0, 24.0)
+    light = tuple(np.array(p, np.float32) for p in ([-3, 6, -2], [3, 6, 2], [3, 6, -2], e))
+    cam = G.Camera(pos=(0.0, 1.0, -8.0), dir=(0.0, -0.1, 1.0), up=(0.0, 1.0, 0.0), fov=60.0, width=64, height=48)
+    return G.SceneDesc([G._merge(parts)], [G.Instance(0)], [mirror, G.Material(G.EMISSIVE, color=(0, 0, 0), emission=e)],
+                       [light], cam, None, "mirrors")
+
+
+@pytest.mark.gpu
+def test_light_pass_fits_without_spare_room(cuda):
+    """A first light pass that fits with one shadow queue and a cache for its paths alone."""
+    from imbatracer_b200.integrators import GpuScene, VcmIntegrator
+    gs = GpuScene(mirrors())
+    paths = 4000000
+
+    def counts(left=None):
+        vi = VcmIntegrator(gs, "bpt", 64, 48, max_path_len=4, light_path_count=paths)
+        vi.begin_iteration(1)
+        img = vi._image(None)
+        if left is None:
+            vi.light_pass(3, image=img)
+        else:
+            with Filled(left):
+                vi.light_pass(3, image=img)
+                assert N.last_error()[0] == 0
+        assert len(vi.light_vertices()) == 0
+        vi.close()
+        return vi.last_stats[:3].tolist()
+    want = counts()
+    # 276 B a path, one shadow queue of 68, room for a vertex of 112 each.
+    assert counts((276 + 68 + 112) * paths + 64 * MB) == want
