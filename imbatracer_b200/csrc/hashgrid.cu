@@ -42,6 +42,7 @@ struct imbart_hashgrid {
     int* block_sums = nullptr;  // scan scratch
     int block_sums_cap = 0;
     unsigned* state = nullptr;  // 8 words, zero between builds (GridState)
+    bool state_zeroed = false;  // by an earlier build
     float* params = nullptr;    // device: lo[3], hi[3], radius, r^2, cell, inv_cell
     float host_params[10] = {};
     float cell_factor = 2.0f;   // cell size / radius of the current build
@@ -346,10 +347,10 @@ imbart_hashgrid* imbart_hashgrid_create(int device) {
     int prev = 0;
     cudaGetDevice(&prev);
     cudaSetDevice(device);
-    // The parameters, then the builds' state words, zero until the first build.
-    const size_t bytes = sizeof(float) * 16 + sizeof(unsigned) * kStateWords;
-    const bool good = ok(cudaMalloc((void**)&g->params, bytes), "cudaMalloc") &&
-                      ok(zero_now(g->params, bytes), "cudaMemsetAsync");
+    // The parameters, then the builds' state words (zeroed by the first build on its stream: a wait
+    // for the device here would end a graph capture in progress on another thread).
+    const bool good = ok(cudaMalloc((void**)&g->params, sizeof(float) * 16 + sizeof(unsigned) * kStateWords),
+                         "cudaMalloc");
     cudaSetDevice(prev);
     if (!good) { cudaFree(g->params); delete g; return nullptr; }
     g->state = reinterpret_cast<unsigned*>(g->params + 16);
@@ -382,10 +383,21 @@ int imbart_hashgrid_build(imbart_hashgrid* g, const float* positions, int stride
     if (!grow(&g->sorted, &g->sorted_cap, n) || !grow(&g->place, &g->place_cap, n) ||
         !grow(&g->cell_ends, &g->ends_cap, table_size) || !grow(&g->block_sums, &g->block_sums_cap, n_tiles))
         rc = IMBART_ERR_OUT_OF_MEMORY;
+    if (!rc && !g->state_zeroed) {
+        // Under capture the zeroing is recorded, not done: the next build repeats it.
+        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+        if (!ok(cudaMemsetAsync(g->state, 0, sizeof(unsigned) * kStateWords, st), "cudaMemsetAsync") ||
+            !ok(cudaStreamIsCapturing(st, &capturing), "cudaStreamIsCapturing"))
+            rc = IMBART_ERR_CUDA;
+        g->state_zeroed = !rc && capturing == cudaStreamCaptureStatusNone;
+    }
     if (!rc) {
         launch_build(positions, stride, n, radius, cell_factor, table_size, g->sorted, g->cell_ends, g->params, g->place,
                      g->block_sums, g->state, st);
-        if (!ok(cudaGetLastError(), "hash grid build")) rc = IMBART_ERR_CUDA;
+        if (!ok(cudaGetLastError(), "hash grid build")) {
+            rc = IMBART_ERR_CUDA;
+            g->state_zeroed = false;
+        }
         g->n = n;
         g->table = table_size;
         g->cell_factor = cell_factor;

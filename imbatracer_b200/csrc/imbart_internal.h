@@ -175,18 +175,6 @@ int vcm_estimate_pixel_size(imbart_vcm* v, const imbart_scene* scene, const imba
 inline int float_bits(float f) { union { float f; int i; } u; u.f = f; return u.i; }
 inline float bits_float(int i) { union { float f; int i; } u; u.i = i; return u.f; }
 
-// Zeroes device memory and waits for that alone: a stream of its own, since a wait for the whole
-// device or work on the default stream would end a graph capture in progress on another thread.
-inline cudaError_t zero_now(void* p, size_t bytes) {
-    cudaStream_t st = nullptr;
-    cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-    if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(p, 0, bytes, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaStreamDestroy(st);
-    return e;
-}
-
 // Several arrays in one device allocation, each 256-byte aligned: an allocation costs about
 // 0.34 ms and its release 0.29 whatever the size (B200), so the queues of a new context come as
 // one block per pass instead of one per array. First frames of new contexts: bidirectional,
