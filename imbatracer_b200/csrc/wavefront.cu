@@ -71,6 +71,7 @@ struct imbart_pt_context {
     // Forked form: a second shadow queue, so that a bounce's shadow rays are traced beside the
     // next bounce's closest hits.
     void* fork_block = nullptr;
+    long long fork_cap = 0;                  // its rays: the largest range a forked graph was built for
     float4* srays2 = nullptr;
     int4* shits2 = nullptr;
     int* spixel2 = nullptr;
@@ -91,7 +92,7 @@ void free_ctx_buffers(imbart_pt_context* c) {
     cudaFree(c->block);
     cudaFree(c->fork_block);
     c->block = c->fork_block = nullptr;
-    c->srays2 = nullptr;
+    c->fork_cap = 0;
     c->cap = 0;
 }
 
@@ -290,14 +291,19 @@ int build_range_graph(imbart_pt_context* ctx, const imbart_scene* scene, const i
     const int n_slots = 2 * max_path_len + 2;
     long long* state = ctx->range_state;
     int* counts = reinterpret_cast<int*>(state + n_slots + 2);
-    // As large as the first queue: a later frame's range may be larger than this one's.
-    if (fork && !ctx->srays2 && !ok(realloc_block(&ctx->fork_block, [&](BlockLayout& at) {
-            at(&ctx->srays2, 2 * (size_t)ctx->cap);
-            at(&ctx->shits2, (size_t)ctx->cap);
-            at(&ctx->spixel2, (size_t)ctx->cap);
-            at(&ctx->scontrib2, (size_t)ctx->cap);
-        }), "cudaMalloc"))
-        return IMBART_ERR_OUT_OF_MEMORY;
+    // As large as this range, replaced for a larger one (the graph that named the old one is rebuilt
+    // here): the first queue may be far larger, from frames of the unforked forms.
+    if (fork && ctx->fork_cap < chunk) {
+        ctx->fork_cap = 0;
+        if (!ok(realloc_block(&ctx->fork_block, [&](BlockLayout& at) {
+                at(&ctx->srays2, 2 * (size_t)chunk);
+                at(&ctx->shits2, (size_t)chunk);
+                at(&ctx->spixel2, (size_t)chunk);
+                at(&ctx->scontrib2, (size_t)chunk);
+            }), "cudaMalloc"))
+            return IMBART_ERR_OUT_OF_MEMORY;
+        ctx->fork_cap = chunk;
+    }
     GraphBuilder gb;
     if (!ok(cudaGraphCreate(&gb.graph, 0), "cudaGraphCreate")) return IMBART_ERR_CUDA;
     cudaGraphNode_t main = gb.kernel({}, range_begin_kernel, dim3(1), dim3(64), state, counts, n_slots, total, chunk);

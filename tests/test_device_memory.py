@@ -84,6 +84,29 @@ def test_photon_mapping_holds_no_shadow_rays(cuda):
 
 
 @pytest.mark.gpu
+def test_second_queue_of_the_forked_graph_is_as_large_as_its_frames(cuda):
+    """The forked graph's second shadow queue follows the frames that use it, not the largest frame
+    the context has seen."""
+    from imbatracer_b200.integrators import GpuScene, PathTracer
+    gs = GpuScene(small_mixed_scene())
+    pt = PathTracer(gs, max_path_len=3)
+    lib = N.load()
+
+    def frame(w, h, graphs):
+        N.check(lib.imbart_pt_set_graphs(pt.ctx, graphs), "imbart_pt_set_graphs")
+        pt.render(1, 5, w, h)
+    frame(1024, 1024, 0)
+    frame(16, 16, 1)
+    assert held_by(lambda: frame(32, 32, 2)) <= 16 * MB       # 68 B a path; 71 MB for the large frame's
+    frame(1024, 1024, 2)                                      # and it grows when a larger frame needs it
+    a = pt.render(1, 5, 1024, 1024).cpu().numpy()
+    N.check(lib.imbart_pt_set_graphs(pt.ctx, 0), "imbart_pt_set_graphs")
+    b = pt.render(1, 5, 1024, 1024).cpu().numpy()
+    assert np.abs(a - b).max() <= 6 * 2.0 ** -23 * np.abs(b).max()
+    pt.close()
+
+
+@pytest.mark.gpu
 def test_connections_fit_with_one_shadow_queue(cuda):
     """A camera pass whose shadow rays fit once but not twice."""
     from imbatracer_b200.integrators import GpuScene, VcmIntegrator
