@@ -40,6 +40,7 @@
 #include <climits>
 #include <cmath>
 #include <cstddef>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -1007,7 +1008,12 @@ void give_scratch(int device, char* base, size_t bytes) {
     cudaFree(base);
 }
 
-constexpr long long kBatchPrims = 32ll << 20;   // meshes are built together up to this many primitives
+// Meshes are built together up to this many primitives (IMBART_BUILD_BATCH).
+long long batch_prims() {
+    const char* v = getenv("IMBART_BUILD_BATCH");
+    const long long n = v ? atoll(v) : 0;
+    return n > 0 ? n : 32ll << 20;
+}
 constexpr int kMaxBuildBlocks = 2048;
 
 // Device arrays of a scene build.
@@ -1086,6 +1092,19 @@ int build_error(int code) {
     }
 }
 
+// What a build is given, with the meshes' places in the scene.
+struct SceneInput {
+    const imbart_mesh_desc* meshes;
+    int n_meshes;
+    const imbart_instance_desc* insts;
+    int n_insts;
+    long long total_tris = 0, total_verts = 0;
+    std::vector<long long> vert_first;
+    std::vector<int> vert_count, tri_offset;
+};
+
+int build_batches(const SceneInput& in, long long limit, int device, cudaStream_t st, imbart_scene** out);
+
 int build_scene_gpu(const imbart_mesh_desc* meshes, int n_meshes, const imbart_instance_desc* insts, int n_insts,
                     int device, void* stream, imbart_scene** out, float* build_ms) {
     *out = nullptr;
@@ -1093,20 +1112,22 @@ int build_scene_gpu(const imbart_mesh_desc* meshes, int n_meshes, const imbart_i
         set_error(IMBART_ERR_INVALID_ARGUMENT, "imbart_scene_build_gpu: invalid argument");
         return IMBART_ERR_INVALID_ARGUMENT;
     }
-    long long total_tris = 0, total_verts = 0, max_n = n_insts;
-    std::vector<long long> vert_first(n_meshes);
-    std::vector<int> vert_count(n_meshes), tri_offset(n_meshes);
+    SceneInput in{meshes, n_meshes, insts, n_insts};
+    in.vert_first.resize(n_meshes);
+    in.vert_count.resize(n_meshes);
+    in.tri_offset.resize(n_meshes);
+    long long max_n = n_insts;
     for (int k = 0; k < n_meshes; ++k) {
         const imbart_mesh_desc& m = meshes[k];
         if (!m.vertices || !m.indices || m.n_vertices <= 0 || m.n_tris <= 0) {
             set_error(IMBART_ERR_INVALID_ARGUMENT, "imbart_scene_build_gpu: empty mesh");
             return IMBART_ERR_INVALID_ARGUMENT;
         }
-        vert_first[k] = total_verts;
-        vert_count[k] = m.n_vertices;
-        tri_offset[k] = m.tri_offset;
-        total_verts += m.n_vertices;
-        total_tris += m.n_tris;
+        in.vert_first[k] = in.total_verts;
+        in.vert_count[k] = m.n_vertices;
+        in.tri_offset[k] = m.tri_offset;
+        in.total_verts += m.n_vertices;
+        in.total_tris += m.n_tris;
         max_n = std::max<long long>(max_n, m.n_tris);
     }
     for (int i = 0; i < n_insts; ++i)
@@ -1114,33 +1135,59 @@ int build_scene_gpu(const imbart_mesh_desc* meshes, int n_meshes, const imbart_i
             set_error(IMBART_ERR_BAD_SCENE, "imbart_scene_build_gpu: instance of an unknown mesh");
             return IMBART_ERR_BAD_SCENE;
         }
-    if (total_tris >= (1ll << 30) || max_n >= (1ll << 29)) {
+    if (in.total_tris >= (1ll << 30) || max_n >= (1ll << 29)) {
         set_error(IMBART_ERR_LIMIT, "imbart_scene_build_gpu: scene too large");
         return IMBART_ERR_LIMIT;
     }
-    // Batches of consecutive meshes; the last one takes the instances too.
-    std::vector<int> batch_end;
-    long long cap = 0, in_batch = 0;
-    int max_seg = 1, batch_first = 0;
-    for (int k = 0; k < n_meshes; ++k) {
-        if (in_batch > 0 && in_batch + meshes[k].n_tris > kBatchPrims) {
-            batch_end.push_back(k);
-            cap = std::max(cap, in_batch);
-            max_seg = std::max(max_seg, k - batch_first);
-            batch_first = k;
-            in_batch = 0;
-        }
-        in_batch += meshes[k].n_tris;
-    }
-    batch_end.push_back(n_meshes);
-    cap = std::max(cap, in_batch + n_insts);
-    max_seg = std::max(max_seg, n_meshes - batch_first + 1);
-    const bool single = batch_end.size() == 1 && cap <= kBatchPrims;
     int prev = 0;
     cudaGetDevice(&prev);
     if (!ck(cudaSetDevice(device), "cudaSetDevice")) return IMBART_ERR_CUDA;
-    cudaStream_t st = (cudaStream_t)stream;
     const auto t0 = std::chrono::steady_clock::now();
+    const int code = imbart_last_error();
+    const std::string msg = imbart_last_error_string();
+    int rc = build_batches(in, batch_prims(), device, (cudaStream_t)stream, out);
+    if (rc == IMBART_ERR_OUT_OF_MEMORY) {
+        // Building the meshes together takes up to 540 B a triangle; one after another they take the
+        // records (128 B) and the scratch of the largest (281 B).
+        (void)cudaGetLastError();
+        release_build_scratch();
+        rc = build_batches(in, 0, device, (cudaStream_t)stream, out);
+        if (rc == 0) set_error(code, msg);
+    }
+    if (rc == 0 && build_ms)
+        *build_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    cudaSetDevice(prev);
+    return rc;
+}
+
+// Builds the scene in batches of consecutive meshes of at most `limit` primitives (or one mesh); the
+// last one takes the instances too where they fit. A scene of one batch goes into one allocation.
+int build_batches(const SceneInput& in, long long limit, int device, cudaStream_t st, imbart_scene** out) {
+    const imbart_mesh_desc* meshes = in.meshes;
+    const imbart_instance_desc* insts = in.insts;
+    const int n_meshes = in.n_meshes, n_insts = in.n_insts;
+    const long long total_tris = in.total_tris, total_verts = in.total_verts;
+    const std::vector<long long>& vert_first = in.vert_first;
+    const std::vector<int>&vert_count = in.vert_count, &tri_offset = in.tri_offset;
+    std::vector<int> batch_end;
+    long long cap = 0, in_batch = 0;
+    int max_seg = 1, batch_first = 0;
+    auto close_batch = [&](int k) {
+        batch_end.push_back(k);
+        cap = std::max(cap, in_batch);
+        max_seg = std::max(max_seg, k - batch_first);
+        batch_first = k;
+        in_batch = 0;
+    };
+    for (int k = 0; k < n_meshes; ++k) {
+        if (in_batch > 0 && in_batch + meshes[k].n_tris > limit) close_batch(k);
+        in_batch += meshes[k].n_tris;
+    }
+    if (in_batch + n_insts > limit) close_batch(n_meshes);
+    batch_end.push_back(n_meshes);
+    cap = std::max(cap, in_batch + n_insts);
+    max_seg = std::max(max_seg, n_meshes - batch_first + 1);
+    const bool single = batch_end.size() == 1;
     // Wide nodes: at most one per binary internal node, plus one per mesh (and the top).
     const long long node_cap = total_tris + n_insts + n_meshes + 2;
     size_t temp_bytes = 0;
@@ -1286,14 +1333,11 @@ int build_scene_gpu(const imbart_mesh_desc* meshes, int n_meshes, const imbart_i
         *out = scene_adopt_device_arrays(device, block, nodes, hs.wide_count, hs.wide_count - hs.bottom_nodes, tris,
                                          hs.tri_count, winsts, n_insts, error_flags, hs.bottom_nodes, direct_root,
                                          direct_inst);
-        if (build_ms)
-            *build_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
     } else {
         cudaFree(block);
         if (!single) { cudaFree(nodes); cudaFree(tris); cudaFree(winsts); cudaFree(error_flags); }
         if (!rc) rc = imbart_last_error() ? imbart_last_error() : IMBART_ERR_CUDA;
     }
-    cudaSetDevice(prev);
     return rc;
 }
 

@@ -795,8 +795,10 @@ struct imbart_instance_desc {
 /* Builds a scene entirely on the GPU (PLOC clustering over Morton-sorted primitives, a
  * surface-area leaf pass, a collapse into the compressed 8-wide layout) and returns it ready
  * for imbart_trace and the renderers, like imbart_scene_from_node2 (unmasked). One BVH per
- * mesh, a top-level BVH over the instances. Synchronizes `stream`; build_ms (may be NULL)
- * receives the wall time. NULL on error (imbart_last_error). */
+ * mesh, a top-level BVH over the instances. Meshes are built together up to 32M primitives
+ * (environment: IMBART_BUILD_BATCH), one after another where device memory does not suffice.
+ * Synchronizes `stream`; build_ms (may be NULL) receives the wall time. NULL on error
+ * (imbart_last_error). */
 imbart_scene* imbart_scene_build_gpu(const imbart_mesh_desc* meshes, int n_meshes,
                                      const imbart_instance_desc* instances, int n_instances, int device,
                                      void* stream, float* build_ms);

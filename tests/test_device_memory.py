@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from imbatracer_b200 import native as N
+from imbatracer_b200 import scene as S
 from imbatracer_b200 import scenegen as G
 from tests.test_pt import small_mixed_scene
 
@@ -172,3 +173,35 @@ def test_light_pass_fits_without_spare_room(cuda):
     want = counts()
     # 276 B a path, one shadow queue of 68, room for a vertex of 112 each.
     assert counts((276 + 68 + 112) * paths + 64 * MB) == want
+
+
+@pytest.mark.gpu
+def test_scene_build_fits_mesh_by_mesh(cuda):
+    """48 meshes of 328 k triangles: built together they need 540 B a triangle, one after another
+    the records (128 B a triangle) and the scratch of one mesh."""
+    rng = np.random.default_rng(3)
+    v, f = G.displaced_sphere(rng, 7, (0, 0, 0), 1.0)
+    mesh = S.Mesh(v, np.concatenate([f, np.zeros((len(f), 1), np.int32)], 1).astype(np.int32))
+    meshes, insts = [mesh] * 48, []
+    for k in range(48):
+        m = np.eye(4, dtype=np.float32)
+        m[:3, 3] = (3.0 * (k % 7), 3.0 * (k // 7), 0.0)
+        insts.append(S.Instance(k, m))
+    n = sum(m.triangle_count for m in meshes)
+    rays = G.random_rays(rng, 4000, [-2] * 3, [20, 20, 2])
+    from tests.test_gpu_build import trace
+
+    def hits(left=None):
+        if left is None:
+            ds = S.DeviceScene.build_gpu(meshes, insts)
+        else:
+            with Filled(left):
+                ds = S.DeviceScene.build_gpu(meshes, insts)
+                assert N.last_error()[0] == 0
+        assert ds.info.triangles == n
+        out = trace(ds, rays)[0]
+        ds.close()
+        return out
+    want = hits()
+    assert (want["tri_id"] >= 0).sum() > 100
+    assert np.array_equal(want, hits(int(200 * n)))

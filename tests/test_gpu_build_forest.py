@@ -52,6 +52,21 @@ def records(ds, which, count, size):
 @pytest.mark.gpu
 @pytest.mark.parametrize("name", ["one", "tiny trees", "edges", "coinciding", "large"])
 def test_forest_build_and_refit(cuda, name):
+    build_and_refit(name)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,limit", [("one", 1), ("tiny trees", 500), ("tiny trees", 100000), ("edges", 3000),
+                                        ("edges", 4512), ("coinciding", 1500)])
+def test_forest_in_batches(cuda, monkeypatch, name, limit):
+    """Scenes above the batch limit: meshes above it alone, instances in the last batch or, where
+    they do not fit there, in one of their own; the same hits, and refits of records and nodes that
+    several batches wrote."""
+    monkeypatch.setenv("IMBART_BUILD_BATCH", str(limit))
+    build_and_refit(name)
+
+
+def build_and_refit(name):
     meshes, instances = forest(name)
     n_tris = sum(m.triangle_count for m in meshes)
     ds = S.DeviceScene.build_gpu(meshes, instances)
