@@ -385,15 +385,24 @@ struct PlocArrays {
     int2* sums;             // per block
 };
 constexpr int kKeep = -1, kGone = -2;
+constexpr int kPlainRounds = 128;   // rounds by nearest neighbours; ordinary scenes take about 35
 constexpr int kSolo = 1024; // clusters from which one block goes on alone (no barriers)
 constexpr int kOwn = kBlock - 2 * kRadius;   // clusters of a tile: its neighbours within kRadius fill the block
 
 // 3. PLOC. Each block owns a contiguous run of clusters and takes it in tiles of kOwn: boxes of the
 // tile and 32 positions on either side in shared memory, nearest neighbours of the tile and 16
 // positions on either side, one per thread (so that a merge is known to be mutual without another
-// barrier), then
-// after a barrier the compaction into the other buffers at the blocks' scanned offsets. Two
-// barriers a round; below kSolo clusters one block goes on alone.
+// barrier), then after a barrier the compaction into the other buffers at the blocks' scanned
+// offsets. Two barriers a round; below kSolo clusters one block goes on alone.
+//
+// Rounds are few as long as many clusters merge in each. Of equally near neighbours a cluster takes
+// the one it shares an even-odd pair of positions with, then the smallest position: coinciding or
+// evenly spaced primitives then pair up and halve every round (the smallest position alone made all
+// but the first cluster point at ever smaller ones, one merge and one more level a round). Distances
+// that grow along the order do the same without ties, so after kPlainRounds the pairs of positions
+// merge as they stand, even-odd and odd-even in turn. Measured (B200): 30,000 triangles at growing
+// spacings 84 -> 3 ms; the kernel over the instanced scene's 104 k triangles 394 -> 388 us, over 8
+// and 100 spheres of 5,120 297 -> 307 and 676 -> 687 us.
 __global__ void __launch_bounds__(kBlock) ploc_kernel(Forest f, PlocArrays p, BuildState* st) {
     constexpr int kHalo = 2 * kRadius;
     __shared__ float4 sb4[kOwn + 2 * kHalo];     // staged boxes: low corner, high x
@@ -415,7 +424,8 @@ __global__ void __launch_bounds__(kBlock) ploc_kernel(Forest f, PlocArrays p, Bu
     if (!grid_barrier(st, target)) return;
     int m = f.n, made = 0, cur = 0;
     bool solo = gridDim.x == 1;
-    while (m > f.n_seg) {
+    for (int round = 0; m > f.n_seg; ++round) {
+        const bool plain = round >= kPlainRounds;
         if (!solo && m <= kSolo) {
             if (blockIdx.x != 0) return;
             solo = true;
@@ -449,9 +459,7 @@ __global__ void __launch_bounds__(kBlock) ploc_kernel(Forest f, PlocArrays p, Bu
                 const float4 a4 = sb4[c];
                 const float2 a2 = sb2[c];
                 float best = FLT_MAX;
-#pragma unroll 8
-                for (int o = 0; o < 2 * kRadius; ++o) {
-                    const int j = c + (o < kRadius ? o - kRadius : o - kRadius + 1);
+                auto consider = [&](int j) {
                     const float4 b4 = sb4[j];
                     const float2 b2 = sb2[j];
                     // half_area of the union
@@ -459,7 +467,18 @@ __global__ void __launch_bounds__(kBlock) ploc_kernel(Forest f, PlocArrays p, Bu
                     const float dy = fmaxf(fmaxf(a2.x, b2.x) - fminf(a4.y, b4.y), 0.0f);
                     const float dz = fmaxf(fmaxf(a2.y, b2.y) - fminf(a4.z, b4.z), 0.0f);
                     const float d = ss[j] == seg ? dx * (dy + dz) + dy * dz : FLT_MAX;
-                    if (d < best) { best = d; bj = j; }   // ties: the smaller position
+                    if (d < best) { best = d; bj = j; }   // of equal ones the first considered
+                };
+                // Tiles start at even positions: c has its position's parity, its pair is c ^ 1.
+                const int pair = c ^ 1;
+                if (plain) {
+                    consider((round & 1) ? 2 * c - pair : pair);
+                } else {
+                    consider(pair);
+                    consider(2 * c - pair);
+#pragma unroll 10
+                    for (int o = 0; o < 2 * kRadius - 2; ++o)
+                        consider(c + (o < kRadius - 1 ? o - kRadius : o - kRadius + 3));
                 }
             }
             snn[tid] = bj;
@@ -480,7 +499,9 @@ __global__ void __launch_bounds__(kBlock) ploc_kernel(Forest f, PlocArrays p, Bu
             if (!grid_barrier(st, target)) return;
             block_prefix(p.sums, blocks, blockIdx.x, before, total);
         }
-        if (total.y <= 0) {
+        // Pairs of one parity may all cross segments, so a plain round may pass without a merge; two
+        // of them at least halve every segment that is longer than two.
+        if (plain ? round >= kPlainRounds + 2 * 40 : total.y <= 0) {
             if (tid == 0) atomicExch(&st->error, kErrProgress);
             return;   // every block sees the same total
         }

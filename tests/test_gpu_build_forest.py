@@ -132,3 +132,64 @@ def test_scratch_between_builds(cuda):
     for t in threads:
         t.join()
     assert wrong == []
+
+
+def slivers(x):
+    """A small triangle at each x along an axis, all alike."""
+    v = np.zeros((len(x), 3, 3))
+    v[:, :, 0] = np.asarray(x)[:, None]
+    v += np.array([[0, 0, 0], [0.25, 0, 0], [0, 0.25, 0.125]])
+    n = len(x)
+    idx = np.concatenate([np.arange(3 * n).reshape(n, 3), np.zeros((n, 1), int)], 1)
+    return S.Mesh(v.reshape(-1, 3).astype(np.float32), idx.astype(np.int32))
+
+
+def levels(ds, root):
+    """Levels of wide nodes below `root`."""
+    nodes = records(ds, 0, int(ds.info.wide_nodes), 80)
+    internal = np.unpackbits(nodes[:, 15:16], axis=1).sum(1).astype(np.int64)
+    base = nodes[:, 16:20].copy().view(np.uint32)[:, 0].astype(np.int64)
+    at, n = np.array([root]), 0
+    while len(at):
+        n += 1
+        at = np.concatenate([np.arange(base[i], base[i] + internal[i]) for i in at])
+    return n
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,n", [("coinciding", 1500), ("points", 5000), ("even", 4096), ("even", 30011),
+                                    ("growing", 30000)])
+def test_trees_of_tied_neighbours_are_shallow(cuda, name, n):
+    """Every round adds at most one level and takes one pass over the clusters. Equally near
+    neighbours pair up, so coinciding, extentless and evenly spaced triangles halve every round or
+    nearly; spacings that grow along the row (no ties, each nearest to the one before) merge one pair
+    a round until the positions pair up as they stand, after 128 rounds. Half as many rounds as
+    triangles took 100 ms, these take 3."""
+    if name == "points":
+        m = slivers(np.zeros(n))
+        mesh = S.Mesh(np.repeat(np.arange(n, dtype=np.float32), 3)[:, None] * np.float32([1, 0, 0]), m.indices)
+    else:
+        mesh = slivers({"coinciding": np.zeros(n), "even": np.arange(n), "growing": np.arange(n) ** 2 / 1024.0}[name])
+    ds = S.DeviceScene.build_gpu([soup(np.random.default_rng(1), 3), mesh], [S.Instance(0), S.Instance(1)])
+    halvings = int(np.ceil(np.log2(n)))
+    assert levels(ds, 1) <= (2 * halvings if name != "growing" else 128 + 2 * halvings)
+    if name == "growing":
+        times = []
+        for _ in range(3):
+            again = S.DeviceScene.build_gpu([soup(np.random.default_rng(1), 3), mesh], [S.Instance(0), S.Instance(1)])
+            times.append(again.build_ms)
+            again.close()
+        assert min(times) < 30.0
+    if name != "points":
+        rng = np.random.default_rng(2)
+        pick = rng.integers(0, n, 500)
+        target = mesh.vertices.reshape(n, 3, 3)[pick].mean(1)
+        org = target + rng.normal(size=target.shape)
+        from imbatracer_b200 import native as N
+        rays = np.zeros(500, N.RAY_DTYPE)
+        rays["org"][:, :3], rays["dir"][:, :3], rays["dir"][:, 3] = org, target - org, 3.0e38
+        meshes = [soup(np.random.default_rng(1), 3), mesh]
+        want = O.trace_brute(meshes, [S.Instance(0), S.Instance(1)], np.array([0, 3], np.int32), rays)
+        got, _ = trace(ds, rays)
+        assert (want["tri_id"] >= 0).sum() > 400 and H.hits_equal(want, got).all()
+    ds.close()
