@@ -198,10 +198,11 @@ struct Collapse {
             }
             c.cost[0] = nd.box.half_area() + c.cost[width - 1];
             c.split[0] = 0;
-            // The entry counts below the full width may prefer a wide node of its own; the full
-            // width's split stays, it is how that wide node takes its children.
+            // The entry counts below the full width may prefer a wide node of its own (not where both
+            // cost the same, as among boxes without area: that filled no nodes); the full width's
+            // split stays, it is how that wide node takes its children.
             for (int m = 2; m < width; ++m)
-                if (c.cost[0] <= c.cost[m - 1]) { c.cost[m - 1] = c.cost[0]; c.split[m - 1] = 0; }
+                if (c.cost[0] < c.cost[m - 1]) { c.cost[m - 1] = c.cost[0]; c.split[m - 1] = 0; }
         }
     }
 

@@ -368,7 +368,7 @@ __device__ __forceinline__ void choose_collapse(const Forest& f, int k, int l, i
         cost[0] = a + cost[7];
 #pragma unroll
         for (int m = 2; m < 8; ++m)
-            if (cost[0] <= cost[m - 1]) { cost[m - 1] = cost[0]; split[m - 1] = 0; }
+            if (cost[0] < cost[m - 1]) { cost[m - 1] = cost[0]; split[m - 1] = 0; }
     }
     for (int m = 0; m < 7; ++m) out[m] = cost[m];
     uint32_t w[2] = {0u, 0u};

@@ -3,6 +3,7 @@ parent, and the node slots filled (opening the child of largest area left 4.2-4.
 import numpy as np
 import pytest
 
+from imbatracer_b200 import scene as S
 from tests import helpers as H
 
 
@@ -23,3 +24,16 @@ def test_collapse_is_a_tree_with_filled_nodes(name, width, fill):
         np.ascontiguousarray(insts).view(np.uint8).reshape(-1, 64))
     assert (internal + leaves).max() <= width
     assert (internal + leaves).mean() >= fill
+
+
+@pytest.mark.parametrize("width,most", [(8, 0.15), (4, 0.3)])
+def test_collapse_of_extentless_geometry(width, most):
+    """Boxes without area cost nothing either way: their nodes are filled all the same, instead of one
+    wide node for every binary one (0.76 n of them)."""
+    n = 3000
+    v = np.zeros((3 * n, 3), np.float32)
+    v[:, 0] = np.repeat(np.arange(n), 3)
+    idx = np.concatenate([np.arange(3 * n).reshape(n, 3), np.zeros((n, 1), int)], 1).astype(np.int32)
+    td = S.build_traversal_data([S.Mesh(v, idx)], [S.Instance(0)])
+    nodes, tris = H.wide_arrays(td, width)[:2]
+    assert len(tris) == n and len(nodes) <= most * n

@@ -172,6 +172,8 @@ def test_trees_of_tied_neighbours_are_shallow(cuda, name, n):
         mesh = slivers({"coinciding": np.zeros(n), "even": np.arange(n), "growing": np.arange(n) ** 2 / 1024.0}[name])
     ds = S.DeviceScene.build_gpu([soup(np.random.default_rng(1), 3), mesh], [S.Instance(0), S.Instance(1)])
     halvings = int(np.ceil(np.log2(n)))
+    if name == "points":
+        assert ds.info.wide_nodes <= 0.3 * n           # no box has an area; a node per binary one: n / 2
     assert levels(ds, 1) <= (2 * halvings if name != "growing" else 128 + 2 * halvings)
     if name == "growing":
         times = []
