@@ -1499,6 +1499,7 @@ __global__ void __launch_bounds__(kBlock) refit_up_kernel(WideNode* nodes, int f
                 up = p;
             }
         }
+        __syncwarp();    // the shuffle alone would not order the other lanes' reads behind lane 0's fence
         n = __shfl_sync(full, up, 0, 8);
         active = n >= 0;
     }
