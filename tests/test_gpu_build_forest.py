@@ -102,17 +102,18 @@ def test_scratch_between_builds(cuda):
     """The scratch kept from one build to the next: smaller and larger scenes after each other, given
     back between builds, and two threads building at once; every build's arrays are the first one's."""
     import threading
+    import torch
     from imbatracer_b200 import native as N
     scenes = [forest(n) for n in ("tiny trees", "one", "large", "edges")]
 
-    def arrays(k):
-        ds = S.DeviceScene.build_gpu(*scenes[k])
+    def arrays(k, stream=None):
+        ds = S.DeviceScene.build_gpu(*scenes[k], stream=stream)
         out = [records(ds, 0, int(ds.info.wide_nodes), 80), records(ds, 1, int(ds.info.triangles), 48)]
         ds.close()
         return out
 
-    def same(k):
-        return all(np.array_equal(a, b) for a, b in zip(first[k], arrays(k)))
+    def same(k, stream=None):
+        return all(np.array_equal(a, b) for a, b in zip(first[k], arrays(k, stream)))
 
     first = [arrays(k) for k in range(4)]
     for k in (1, 2, 0, 3, 2):
@@ -123,7 +124,8 @@ def test_scratch_between_builds(cuda):
 
     def work(order):
         try:
-            wrong.extend(k for k in order if not same(k))
+            stream = torch.cuda.Stream()       # of the thread's own: the builds overlap on the device
+            wrong.extend(k for k in order if not same(k, stream))
         except Exception as e:          # shown by the assertion below
             wrong.append(repr(e))
     threads = [threading.Thread(target=work, args=(o,)) for o in ([0, 1, 2, 3] * 2, [2, 3, 0, 1] * 2)]
