@@ -99,22 +99,24 @@ __global__ void bounds_init_kernel(int* cb, int n) {
 }
 
 // Adds centroids to their segments' bounds (ordered-int atomics). A warp whose primitives all
-// belong to one segment reduces first.
+// belong to one segment reduces first. NaN coordinates stay out: their encoding lies beyond every
+// float's, and bounds that hold one order the segment's primitives along no curve.
 __device__ __forceinline__ void add_centroid(const Box6& b, bool valid, int seg, int* cb) {
     const unsigned full = 0xffffffffu;
     const int s0 = __shfl_sync(full, seg, 0);
     const bool uniform = __all_sync(full, !valid || seg == s0);
     for (int k = 0; k < 3; ++k) {
         const float c = 0.5f * (b.lo[k] + b.hi[k]);
+        const bool in = valid && c == c;
         if (uniform) {
-            const int lo = __reduce_min_sync(full, valid ? f2ord(c) : 0x7fffffff);
-            const int hi = __reduce_max_sync(full, valid ? f2ord(c) : (int)0x80000000);
+            const int lo = __reduce_min_sync(full, in ? f2ord(c) : 0x7fffffff);
+            const int hi = __reduce_max_sync(full, in ? f2ord(c) : (int)0x80000000);
             if ((threadIdx.x & 31) == 0 && lo <= hi) {
                 int* q = cb + 6 * s0 + k;
                 if (lo < __ldcg(q)) atomicMin(q, lo);
                 if (hi > __ldcg(q + 3)) atomicMax(q + 3, hi);
             }
-        } else if (valid) {
+        } else if (in) {
             atomicMin(cb + 6 * seg + k, f2ord(c));
             atomicMax(cb + 6 * seg + 3 + k, f2ord(c));
         }

@@ -197,3 +197,31 @@ def test_trees_of_tied_neighbours_are_shallow(cuda, name, n):
         got, _ = trace(ds, rays)
         assert (want["tri_id"] >= 0).sum() > 400 and H.hits_equal(want, got).all()
     ds.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+def test_a_triangle_without_a_position_leaves_the_tree_as_good(cuda, sign):
+    """NaN vertices (of either sign) stay out of the box that the order along the curve is cut from:
+    rays visit as many nodes of the others' tree as without them."""
+    import torch
+    from imbatracer_b200 import native as N
+    lib = N.load()
+    mesh = soup(np.random.default_rng(4), 20000, 10.0, 0.1)
+    v = np.concatenate([mesh.vertices, np.full((3, 3), np.copysign(np.float32(np.nan), np.float32(sign)))])
+    lost = S.Mesh(v.astype(np.float32), np.concatenate([mesh.indices, [[60000, 60001, 60002, 0]]]).astype(np.int32))
+    rays = G.random_rays(np.random.default_rng(5), 4000, [-10] * 3, [10] * 3)
+    r = torch.from_numpy(rays.view(np.float32).reshape(-1, 8).copy()).cuda()
+    visits, hits = [], []
+    for m in (mesh, lost):
+        ds = S.DeviceScene.build_gpu([m], [S.Instance(0)])
+        h = torch.zeros((len(rays), 4), dtype=torch.int32, device="cuda")
+        counts = torch.zeros(3, dtype=torch.int64, device="cuda")
+        N.check(lib.imbart_trace_stats(ds.handle, N.ptr(r), N.ptr(h), len(rays), N.TRACE_CLOSEST, N.ptr(counts), None),
+                "imbart_trace_stats")
+        torch.cuda.synchronize()
+        visits.append(int(counts[0]))
+        hits.append(h.cpu().numpy())
+        ds.close()
+    assert np.array_equal(hits[0], hits[1]) and (hits[0][:, 0] >= 0).sum() > 500
+    assert visits[1] <= 1.1 * visits[0], visits
