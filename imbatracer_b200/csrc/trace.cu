@@ -167,10 +167,12 @@ constexpr int kFirstCoopVariant = 11; // 11..17: the shapes with the cooperative
 // frame's ray sets of the instanced scene: camera / secondary / shadow rays +2 / +9 / +10 % over
 // the best per-lane shapes). Incoherent closest hits: 128 x 7, refill at 8 idle lanes (1 M random
 // rays over 201 instances 0.90 ms at 8, 0.89 at 4 and 6, 0.93 at 12, 1.24 at 24; over one mesh
-// 0.181 at 8 and 12, 0.187 at 4; the 256 x 3 shape is 1 % behind on each). Any hit: 256 x 3 at 8
-// (a 1080p frame of the instanced scene 18.26 ms; 18.30 with 128 x 7, which is 4 % ahead on
-// 2 M shadow rays over one masked mesh). Camera rays: 256 x 3 at 24 (the frame 18.20 ms; 18.26
-// at 32, 18.56 at 16).
+// 0.181 at 8 and 12, 0.187 at 4; the 256 x 3 shape is 1 % behind on each). Camera rays: 256 x 3 at
+// 24 (a 1080p frame of the instanced scene 18.20 ms; 18.26 at 32, 18.56 at 16). Any hit: 256 x 3 at
+// 8, the shape before the others changed. Three runs each against 128 x 7: 2 M shadow rays over one
+// masked mesh 404.7 and 388.6 us, a 512 x 512 frame 479.2 and 461.3, the 1080p frame 18.36 and
+// 18.32 ms, a VCM iteration at 720p 11.04 and 10.98, a small bidirectional frame 1,056 and 1,063 us:
+// the autotuner may pick 128 x 7, a default of its own for masked rays is still to be tried.
 struct TraceConfig {
     int variant, refill, postpone, variant_any;
     int refill_any, variant_coh, refill_coh;
