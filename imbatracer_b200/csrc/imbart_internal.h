@@ -112,15 +112,24 @@ long long launches_total();
 // `count_ptr` (optional): device-resident ray count, `count` being its upper bound.
 // `work` (optional): the persistent kernel's (next, done) counter pair, zeroed, owned by the
 // caller (a launch inside a CUDA graph keeps its own); otherwise one of the device's ring.
+// `caller`: the stream that this launch's work belongs to where it is not `stream` itself (a side
+// stream of the same pass; trace_groups).
+inline void* const kOwnStream = reinterpret_cast<void*>(~(uintptr_t)0);
 int launch_trace_internal(const imbart_scene* scene, const void* rays, void* hits, float* v_out, int count,
                           int flags, void* stream, unsigned long long* stats, const int* roots = nullptr,
-                          const int* count_ptr = nullptr, int* work = nullptr);
+                          const int* count_ptr = nullptr, int* work = nullptr, void* caller = kOwnStream);
 
 // Adds one traversal launch (as launch_trace_internal with count_ptr and work) to `graph`
-// after `deps`, under the configuration in force; `count` > 0.
+// after `deps`, under the configuration in force; `count` > 0. groups: the trace_groups() it is
+// sized for.
 int add_trace_node(cudaGraph_t graph, const cudaGraphNode_t* deps, int n_deps, cudaGraphNode_t* node,
                    const imbart_scene* scene, const void* rays, void* hits, int count, int flags,
-                   const int* count_ptr, int* work);
+                   const int* count_ptr, int* work, int groups);
+
+// Notes traversal work of `stream` on the device and returns how many streams had some there in
+// the last 50 ms, this one among them: how many parts short launches leave the device in (1 for a
+// program of one stream). Only speed depends on it.
+int trace_groups(int device, void* stream);
 
 // The traversal configuration in force (variant, refill, postpone, any-hit variant and refill,
 // coherent variant and refill, triangle batches of the three classes): a launch recorded in a

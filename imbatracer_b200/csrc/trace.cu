@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <cfloat>
 #include <climits>
 #include <cstring>
@@ -244,11 +245,43 @@ const void* simple_kernel(bool any, bool masked) {
     return (const void*)trace_kernel<false, false, kStats>;
 }
 
+// Streams that traversal work was given to, by device, with the time of the last. The handles are
+// compared, never used; a thread's default stream counts as the thread's. A program that alternates
+// between streams without overlapping them is taken for a concurrent one for 50 ms, and its short
+// launches get what those of a concurrent one get.
+constexpr int kMaxGroups = 32;
+constexpr long long kGroupWindowNs = 50000000;
+struct GroupTable {
+    std::mutex m;
+    struct { const void* key; long long at; } entry[kMaxGroups] = {};
+    int used = 0;
+};
+GroupTable g_groups[16];
+
+int note_group(int device, cudaStream_t stream) {
+    if (device < 0 || device >= 16) return kMaxGroups;
+    thread_local char own;
+    const void* key = stream == cudaStreamPerThread ? (const void*)&own : (const void*)stream;
+    const long long now = std::chrono::duration_cast<std::chrono::nanoseconds>(
+                              std::chrono::steady_clock::now().time_since_epoch()).count();
+    GroupTable& t = g_groups[device];
+    std::lock_guard<std::mutex> lk(t.m);
+    int at = -1, oldest = 0, busy = 0;
+    for (int i = 0; i < t.used; ++i) {
+        if (t.entry[i].key == key) at = i;
+        else if (now - t.entry[i].at < kGroupWindowNs) ++busy;
+        if (t.entry[i].at < t.entry[oldest].at) oldest = i;
+    }
+    if (at < 0) at = t.used < kMaxGroups ? t.used++ : oldest;
+    t.entry[at] = {key, now};
+    return std::min(busy + 1, kMaxGroups);
+}
+
 // The launch of one traversal query (kernel, grid, block and parameters) under the current
 // configuration; false with the error set on invalid arguments. `count` = 0: nothing to launch.
 bool trace_spec(const imbart_scene* s, const imbart_ray* rays, imbart_hit* hits, float* v_out, int count, int flags,
-                unsigned long long* stats, const int* roots, const int* count_ptr, int* work_override, TraceParams& p,
-                LaunchSpec& spec) {
+                unsigned long long* stats, const int* roots, const int* count_ptr, int* work_override, int groups,
+                bool recorded, TraceParams& p, LaunchSpec& spec) {
     if (!s || (!rays && count > 0) || (!hits && count > 0) || count < 0 || (roots && s->info.masked)) {
         set_error(IMBART_ERR_INVALID_ARGUMENT, "imbart_trace: invalid argument");
         return false;
@@ -264,6 +297,7 @@ bool trace_spec(const imbart_scene* s, const imbart_ray* rays, imbart_hit* hits,
     p.count = count;
     p.roots = roots;
     p.count_ptr = count_ptr;
+    p.groups = groups;
     p.direct_root = roots ? -1 : s->direct_root;
     p.direct_inst = s->direct_inst;
     p.error_flags = s->error_flags;
@@ -272,7 +306,11 @@ bool trace_spec(const imbart_scene* s, const imbart_ray* rays, imbart_hit* hits,
     const bool coherent = !any && (flags & IMBART_TRACE_COHERENT) != 0;
     const bool masked = s->info.masked != 0;
     const TraceConfig cfg = current_config();
-    const int variant = any ? cfg.variant_any : coherent ? cfg.variant_coh : cfg.variant;
+    int variant = any ? cfg.variant_any : coherent ? cfg.variant_coh : cfg.variant;
+    // A recorded launch is sized for its queue's bound, and beside other frames the 1,036 blocks of
+    // 128 x 7, most of them without rays, cost more than the 444 of 256 x 3: 16 frames of 128 x 128
+    // of the instanced scene at once 2.01 and 1.59 ms, of 256 x 192 4.54 and 3.61.
+    if (recorded && groups > 1 && variant == 17) variant = 11;
     const int refill = any ? cfg.refill_any : coherent ? cfg.refill_coh : cfg.refill;
     if (variant == 0) {
         const int block = 128;
@@ -308,10 +346,21 @@ bool trace_spec(const imbart_scene* s, const imbart_ray* rays, imbart_hit* hits,
 
 int launch_trace(const imbart_scene* s, const imbart_ray* rays, imbart_hit* hits, float* v_out,
                  int count, int flags, cudaStream_t stream, unsigned long long* stats = nullptr,
-                 const int* roots = nullptr, const int* count_ptr = nullptr, int* work_override = nullptr) {
+                 const int* roots = nullptr, const int* count_ptr = nullptr, int* work_override = nullptr,
+                 void* caller = kOwnStream) {
     TraceParams p;
     LaunchSpec spec;
-    if (!trace_spec(s, rays, hits, v_out, count, flags, stats, roots, count_ptr, work_override, p, spec))
+    int groups = 1;
+    if (s && count > 0) {
+        // What a recorded launch will run beside is not known: it takes the warps it can fill.
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) (void)cudaGetLastError();
+        groups = capture == cudaStreamCaptureStatusNone
+                     ? note_group(s->device, caller == kOwnStream ? stream : (cudaStream_t)caller)
+                     : kMaxGroups;
+    }
+    if (!trace_spec(s, rays, hits, v_out, count, flags, stats, roots, count_ptr, work_override, groups, false, p,
+                    spec))
         return imbart_last_error() ? imbart_last_error() : IMBART_ERR_CUDA;
     if (!spec.func) return 0;
     void* args[] = {&p};
@@ -466,18 +515,20 @@ void dropin_host(bool any, int root, imbart_node4* nodes, imbart_instance_node* 
 
 int launch_trace_internal(const imbart_scene* scene, const void* rays, void* hits, float* v_out, int count,
                           int flags, void* stream, unsigned long long* stats, const int* roots,
-                          const int* count_ptr, int* work) {
+                          const int* count_ptr, int* work, void* caller) {
     return launch_trace(scene, reinterpret_cast<const imbart_ray*>(rays), reinterpret_cast<imbart_hit*>(hits), v_out,
-                        count, flags, (cudaStream_t)stream, stats, roots, count_ptr, work);
+                        count, flags, (cudaStream_t)stream, stats, roots, count_ptr, work, caller);
 }
+
+int trace_groups(int device, void* stream) { return note_group(device, (cudaStream_t)stream); }
 
 int add_trace_node(cudaGraph_t graph, const cudaGraphNode_t* deps, int n_deps, cudaGraphNode_t* node,
                    const imbart_scene* scene, const void* rays, void* hits, int count, int flags,
-                   const int* count_ptr, int* work) {
+                   const int* count_ptr, int* work, int groups) {
     TraceParams p;
     LaunchSpec spec;
     if (!trace_spec(scene, reinterpret_cast<const imbart_ray*>(rays), reinterpret_cast<imbart_hit*>(hits), nullptr,
-                    count, flags, nullptr, nullptr, count_ptr, work, p, spec))
+                    count, flags, nullptr, nullptr, count_ptr, work, groups, true, p, spec))
         return imbart_last_error() ? imbart_last_error() : IMBART_ERR_CUDA;
     if (!spec.func) {
         set_error(IMBART_ERR_INVALID_ARGUMENT, "add_trace_node: empty launch");

@@ -55,6 +55,8 @@ struct TraceParams {
     // persistent variant
     int* __restrict__ work;                 // [0]: next ray index, [1]: finished warps (self-resetting)
     int total_warps;                        // warps in the launch
+    int part_warps;                         // of these, the caller's part of the device
+    int groups;                             // callers that the launch is sized for (trace_groups)
     int refill_lanes;                       // refill a warp's idle lanes once this many are idle
     int postpone_lanes;                     // postpone triangle tests while fewer lanes would test
     int tri_batch;                          // per-lane kernels: triangles a lane tests per loop trip
@@ -84,6 +86,10 @@ constexpr int kWaitEnter = 8, kWaitPairs = 16, kWaitReady = 8;
 // longest ray bounds such a launch, and a warp with fewer rays passes through its trips sooner:
 // 2,049 rays 47 -> 35 us, 8,000 57 -> 47 us, 20,000 58 -> 55 us. Above that the warps are better
 // filled (50,000 rays, share 15: 72 -> 73 us; 201 instances 194 -> 199 us).
+// Launches of several callers at once (the reference's tile threads, a context per stream) need
+// the warps filled instead, so each spreads its rays over its part of the resident warps only (the
+// part's warps that come first take them all): 16 streams of 8,000 rays over 201 instances ran at 123 M rays/s with
+// every launch spread over all warps, at 552 M before there was any spreading.
 constexpr int kShortShare = 8;
 
 constexpr uint32_t kEntryTri = 3u;      // triangle group (postponed): x = prim base, y = prim mask
@@ -521,8 +527,8 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) trace_persistent(TracePara
     r.Sx = r.Sy = r.Sz = 0.0f;
     r.kx = r.ky = r.kz = 0;
     const int count = p.count_ptr ? min(__ldg(p.count_ptr), p.count) : p.count;
-    // Short queues (kShortShare): lanes beyond the warp's share of the rays stay out.
-    const int share = (int)(((long long)count + p.total_warps - 1) / p.total_warps);
+    // Short queues (kShortShare): lanes beyond a warp's share of the rays stay out.
+    const int share = (int)(((long long)count + p.part_warps - 1) / p.part_warps);
     if (kCoop && share <= kShortShare && (int)lane >= share) ray = count;
 
     auto push = [&](uint32_t x, uint32_t y) -> bool {

@@ -41,12 +41,15 @@ template <int kSlots, bool kFlat, bool kAny, bool kMasked, bool kStats, int kBlo
 LaunchSpec persistent_spec(int count, int device, float share, TraceParams& p) {
     auto k = trace_persistent<kAny, kMasked, kStats, kBlock, kMinBlocks, kSh, kCoop, kSlots, kFlat>;
     const int slots = std::max(1, (int)(max_grid(k, kBlock, device) * share));
-    // Short queues go to as many warps as there are rays, up to the resident ones.
+    // Short queues go to as many warps as there are rays, up to this caller's part of the resident
+    // ones.
     constexpr int kWarps = kBlock / 32;
-    const int spread = std::min(slots, (count + kWarps - 1) / kWarps);
+    const int part = std::max(slots / p.groups, 1);
     const int packed = std::min(slots, (count + kBlock - 1) / kBlock);
+    const int spread = std::max(packed, std::min(part, (count + kWarps - 1) / kWarps));
     const int grid = kCoop && (long long)spread * kWarps * kShortShare >= count ? spread : packed;
-    p.total_warps = grid * (kBlock / 32);
+    p.total_warps = grid * kWarps;
+    p.part_warps = std::min(grid, part) * kWarps;
     return {(const void*)k, dim3(grid), dim3(kBlock)};
 }
 

@@ -951,7 +951,7 @@ int trace_shadows(imbart_vcm* v, const imbart_scene* scene, const VcmParams& p, 
     if (p.algo == kAlgoPpm) return 0;    // no shadow rays
     q.used = true;    // from the first launch on: a pass that fails here still waits for the side stream
     const int rc = launch_trace_internal(scene, q.rays, q.hits, nullptr, bound, IMBART_TRACE_ANY, v->side, nullptr,
-                                         nullptr, p.counts + 1);
+                                         nullptr, p.counts + 1, nullptr, s);
     if (rc) return rc;
     vcm_shadow_kernel<<<(bound + 127) / 128, 128, 0, v->side>>>(p.counts + 1, q.hits, q.pixel, q.contrib, p.image);
     note_launches(1);
