@@ -112,12 +112,10 @@ long long launches_total();
 // `count_ptr` (optional): device-resident ray count, `count` being its upper bound.
 // `work` (optional): the persistent kernel's (next, done) counter pair, zeroed, owned by the
 // caller (a launch inside a CUDA graph keeps its own); otherwise one of the device's ring.
-// `caller`: the stream that this launch's work belongs to where it is not `stream` itself (a side
-// stream of the same pass; trace_groups).
-inline void* const kOwnStream = reinterpret_cast<void*>(~(uintptr_t)0);
+// `groups` (optional): trace_groups() of the pass that the launch belongs to; otherwise `stream`'s.
 int launch_trace_internal(const imbart_scene* scene, const void* rays, void* hits, float* v_out, int count,
                           int flags, void* stream, unsigned long long* stats, const int* roots = nullptr,
-                          const int* count_ptr = nullptr, int* work = nullptr, void* caller = kOwnStream);
+                          const int* count_ptr = nullptr, int* work = nullptr, int groups = 0);
 
 // Adds one traversal launch (as launch_trace_internal with count_ptr and work) to `graph`
 // after `deps`, under the configuration in force; `count` > 0. groups: the trace_groups() it is

@@ -347,17 +347,14 @@ bool trace_spec(const imbart_scene* s, const imbart_ray* rays, imbart_hit* hits,
 int launch_trace(const imbart_scene* s, const imbart_ray* rays, imbart_hit* hits, float* v_out,
                  int count, int flags, cudaStream_t stream, unsigned long long* stats = nullptr,
                  const int* roots = nullptr, const int* count_ptr = nullptr, int* work_override = nullptr,
-                 void* caller = kOwnStream) {
+                 int groups = 0) {
     TraceParams p;
     LaunchSpec spec;
-    int groups = 1;
-    if (s && count > 0) {
+    if (s && groups == 0) {
         // What a recorded launch will run beside is not known: it takes the warps it can fill.
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) (void)cudaGetLastError();
-        groups = capture == cudaStreamCaptureStatusNone
-                     ? note_group(s->device, caller == kOwnStream ? stream : (cudaStream_t)caller)
-                     : kMaxGroups;
+        groups = capture == cudaStreamCaptureStatusNone ? note_group(s->device, stream) : kMaxGroups;
     }
     if (!trace_spec(s, rays, hits, v_out, count, flags, stats, roots, count_ptr, work_override, groups, false, p,
                     spec))
@@ -515,9 +512,9 @@ void dropin_host(bool any, int root, imbart_node4* nodes, imbart_instance_node* 
 
 int launch_trace_internal(const imbart_scene* scene, const void* rays, void* hits, float* v_out, int count,
                           int flags, void* stream, unsigned long long* stats, const int* roots,
-                          const int* count_ptr, int* work, void* caller) {
+                          const int* count_ptr, int* work, int groups) {
     return launch_trace(scene, reinterpret_cast<const imbart_ray*>(rays), reinterpret_cast<imbart_hit*>(hits), v_out,
-                        count, flags, (cudaStream_t)stream, stats, roots, count_ptr, work, caller);
+                        count, flags, (cudaStream_t)stream, stats, roots, count_ptr, work, groups);
 }
 
 int trace_groups(int device, void* stream) { return note_group(device, (cudaStream_t)stream); }

@@ -845,6 +845,7 @@ struct imbart_vcm {
     cudaEvent_t shaded = nullptr;
     int* counts = nullptr;          // 4 per queue (VcmParams::counts), then slot_scan_kernel's `done`
     int* host_counts = nullptr;     // pinned
+    int groups = 1;                 // trace_groups() of the pass
     // iteration state
     int iteration = 0;
     float pm_radius = 0.0f, eta_vc = 0.0f, eta_vm = 0.0f;
@@ -951,7 +952,7 @@ int trace_shadows(imbart_vcm* v, const imbart_scene* scene, const VcmParams& p, 
     if (p.algo == kAlgoPpm) return 0;    // no shadow rays
     q.used = true;    // from the first launch on: a pass that fails here still waits for the side stream
     const int rc = launch_trace_internal(scene, q.rays, q.hits, nullptr, bound, IMBART_TRACE_ANY, v->side, nullptr,
-                                         nullptr, p.counts + 1, nullptr, s);
+                                         nullptr, p.counts + 1, nullptr, v->groups);
     if (rc) return rc;
     vcm_shadow_kernel<<<(bound + 127) / 128, 128, 0, v->side>>>(p.counts + 1, q.hits, q.pixel, q.contrib, p.image);
     note_launches(1);
@@ -1261,6 +1262,7 @@ int imbart_vcm_light_pass_range(imbart_vcm* v, const imbart_scene* scene, const 
         cudaSetDevice(prev);
         return IMBART_ERR_CUDA;
     }
+    v->groups = trace_groups(v->device, s);
     VcmParams p = make_params(v, sh, cam, st, image);
     const int grid = (P + 127) / 128;
     light_gen_kernel<<<grid, 128, 0, s>>>(p, v->d_tiles, (int)tiles.size(), first_path, P, v->l_rays, v->l_rng,
@@ -1289,7 +1291,8 @@ int imbart_vcm_light_pass_range(imbart_vcm* v, const imbart_scene* scene, const 
         }
         const int grid_n = (n + 127) / 128;
         const int n_blocks_n = (n + kScanTile - 1) / kScanTile;
-        rc = launch_trace_internal(scene, v->l_rays, v->l_hits, nullptr, n, IMBART_TRACE_CLOSEST, s, nullptr);
+        rc = launch_trace_internal(scene, v->l_rays, v->l_hits, nullptr, n, IMBART_TRACE_CLOSEST, s, nullptr,
+                                   nullptr, nullptr, nullptr, v->groups);
         if (rc) break;
         n_closest += live;
         if (stores) {
@@ -1458,6 +1461,7 @@ int imbart_vcm_camera_pass_range(imbart_vcm* v, const imbart_scene* scene, const
     }
     good = good && (!casts_shadows(st) || ensure_shadow(v, chunk * per));
     if (!good) { cudaSetDevice(prev); return IMBART_ERR_OUT_OF_MEMORY; }
+    v->groups = trace_groups(v->device, s);
     VcmParams p = make_params(v, sh, cam, st, image);
     long long n_closest = 0, n_shadow = 0, n_waves = 0;
     int rc = 0;
@@ -1469,7 +1473,8 @@ int imbart_vcm_camera_pass_range(imbart_vcm* v, const imbart_scene* scene, const
                                                          v->c_pixel[cur], v->c_rng[cur], v->c_thr[cur], v->c_w[cur]);
         note_launches(1);
         while (n > 0 && !rc) {
-            rc = launch_trace_internal(scene, v->c_rays[cur], v->c_hits, nullptr, n, IMBART_TRACE_CLOSEST, s, nullptr);
+            rc = launch_trace_internal(scene, v->c_rays[cur], v->c_hits, nullptr, n, IMBART_TRACE_CLOSEST, s, nullptr,
+                                       nullptr, nullptr, nullptr, v->groups);
             if (rc) break;
             n_closest += n;
             const int nxt = 1 - cur;
