@@ -5,10 +5,10 @@
 
 #include <algorithm>
 #include <atomic>
-#include <chrono>
 #include <cfloat>
 #include <climits>
 #include <cstring>
+#include <ctime>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -262,8 +262,21 @@ int note_group(int device, cudaStream_t stream) {
     if (device < 0 || device >= 16) return kMaxGroups;
     thread_local char own;
     const void* key = stream == cudaStreamPerThread ? (const void*)&own : (const void*)stream;
-    const long long now = std::chrono::duration_cast<std::chrono::nanoseconds>(
-                              std::chrono::steady_clock::now().time_since_epoch()).count();
+    // The coarse clock (a few ms a tick, a few ns a call): within a tick a thread's earlier answer for
+    // the stream stands, so a launch seldom takes the lock or asks the runtime.
+    timespec ts;
+    clock_gettime(CLOCK_MONOTONIC_COARSE, &ts);
+    const long long now = ts.tv_sec * 1000000000ll + ts.tv_nsec;
+    thread_local struct { const void* key; long long at; int device, groups; } recent[256];
+    auto& r = recent[((uint64_t)(uintptr_t)key * 0x9E3779B97F4A7C15ull) >> 56];
+    if (r.at == now && r.key == key && r.device == device) return r.groups;
+    // What a recorded launch will run beside is not known: it takes the warps it can fill.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) (void)cudaGetLastError();
+    if (capture != cudaStreamCaptureStatusNone) {
+        r = {key, now, device, kMaxGroups};
+        return r.groups;
+    }
     GroupTable& t = g_groups[device];
     std::lock_guard<std::mutex> lk(t.m);
     int at = -1, oldest = 0, busy = 0;
@@ -274,7 +287,8 @@ int note_group(int device, cudaStream_t stream) {
     }
     if (at < 0) at = t.used < kMaxGroups ? t.used++ : oldest;
     t.entry[at] = {key, now};
-    return std::min(busy + 1, kMaxGroups);
+    r = {key, now, device, std::min(busy + 1, kMaxGroups)};
+    return r.groups;
 }
 
 // The launch of one traversal query (kernel, grid, block and parameters) under the current
@@ -350,12 +364,7 @@ int launch_trace(const imbart_scene* s, const imbart_ray* rays, imbart_hit* hits
                  int groups = 0) {
     TraceParams p;
     LaunchSpec spec;
-    if (s && groups == 0) {
-        // What a recorded launch will run beside is not known: it takes the warps it can fill.
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) (void)cudaGetLastError();
-        groups = capture == cudaStreamCaptureStatusNone ? note_group(s->device, stream) : kMaxGroups;
-    }
+    if (s && groups == 0) groups = note_group(s->device, stream);
     if (!trace_spec(s, rays, hits, v_out, count, flags, stats, roots, count_ptr, work_override, groups, false, p,
                     spec))
         return imbart_last_error() ? imbart_last_error() : IMBART_ERR_CUDA;
