@@ -214,7 +214,9 @@ int imbart_scene_get_device_arrays(const imbart_scene* scene, const void** nodes
 enum { IMBART_TRACE_CLOSEST = 0, IMBART_TRACE_ANY = 1, IMBART_TRACE_COHERENT = 2 };
 
 /* Traces `count` rays from DEVICE buffers, stream-ordered on `stream` (a cudaStream_t,
- * NULL = legacy default stream). Returns 0 or an error code; does not synchronize. */
+ * NULL = legacy default stream). Returns 0 or an error code; does not synchronize. A launch of few
+ * rays spreads them over the device while one stream alone is used, over a part of it while several
+ * were in the last 50 ms; recorded in a graph it takes the warps it can fill. */
 int imbart_trace(const imbart_scene* scene, const imbart_ray* rays, imbart_hit* hits,
                  int count, int flags, void* stream);
 
