@@ -40,6 +40,9 @@ def forest(name):
         v = np.tile(m.vertices, (1500, 1))
         idx = np.concatenate([np.arange(4500).reshape(1500, 3), np.zeros((1500, 1), int)], 1).astype(np.int32)
         return [S.Mesh(v, idx), soup(rng, 40)], [S.Instance(0), S.Instance(1)]
+    if name == "many instances":       # fewer blocks an instance than the larger mesh has chunks of vertices
+        meshes = [soup(rng, 3, 0.5, 0.3), soup(rng, 8000, 6.0, 0.1)]
+        return meshes, [placed(rng, int(k in (17, 4321))) for k in range(6000)]
     return [soup(rng, 70000, 10.0, 0.1)], [S.Instance(0)]      # "large": several blocks, one tree
 
 
@@ -50,7 +53,7 @@ def records(ds, which, count, size):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("name", ["one", "tiny trees", "edges", "coinciding", "large"])
+@pytest.mark.parametrize("name", ["one", "tiny trees", "edges", "coinciding", "large", "many instances"])
 def test_forest_build_and_refit(cuda, name):
     build_and_refit(name)
 
